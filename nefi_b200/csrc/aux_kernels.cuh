@@ -251,6 +251,19 @@ __global__ void reduce_grad_kernel(KGrid<T> g, PadMap pm, int ndim, const T* __r
   }
 }
 
+// out[grp] = sum of the fields of the group's shots (spa consecutive shots), in order.
+template <typename T>
+__global__ void group_sum_kernel(const T* __restrict__ per_shot, long long field, int n_shots, int spa,
+                                 T* __restrict__ out) {
+  const int s0 = blockIdx.y * spa, s1 = min(n_shots, s0 + spa);
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < field;
+       i += (long long)gridDim.x * blockDim.x) {
+    T v = per_shot[(long long)s0 * field + i];
+    for (int s = s0 + 1; s < s1; ++s) v = add_rn(v, per_shot[(long long)s * field + i]);
+    out[(long long)blockIdx.y * field + i] = v;
+  }
+}
+
 // Zero the ghost cells of n_fields consecutive fields (a warp per storage row): whole rows
 // outside the grid and the tail [n_last, ld) of every data row. Interior cells are untouched.
 template <typename T>

@@ -1,8 +1,8 @@
 // wave_capi.cu — host drivers and the extern "C" entry points declared in include/nefi_wave.h.
 //
-// The drivers run whole time loops on the caller's stream (one kernel launch per leapfrog step,
-// plus the receiver/adjoint-source kernels), so a forward or adjoint sweep costs one call from
-// the host language. No device memory is allocated here: every buffer comes from the caller.
+// The drivers run whole time loops on the caller's stream (many leapfrog steps per launch where a shot's
+// grid fits the chip, resident2d.cuh, else one kernel launch per step plus the receiver/adjoint-source
+// kernels), so a forward or adjoint sweep costs one call from the host language. No device memory is allocated here: every buffer comes from the caller.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -20,6 +20,7 @@
 #include "kernels.cuh"
 #include "misfit.cuh"
 #include "pml2d.cuh"
+#include "resident2d.cuh"
 #include "stencil2d.cuh"
 #include "stencil3d.cuh"
 
@@ -461,6 +462,293 @@ int launch_step3(const nw_grid* g, const nw::KGrid<T>& kg, const nw::Step3<T>& s
     return ab_ ? FN<T, 1, 2, 8, true>(__VA_ARGS__) : FN<T, 1, 2, 8, false>(__VA_ARGS__);           \
   }()
 
+
+// ---- sweeps of many steps per launch ------------------------------------------------------------
+// CTA clusters of each size that fit the device at once, one CTA per SM (asked once per device).
+int cluster_slots(int size, int* out) {
+  static std::mutex mu;
+  static int slots[64][nw::kMaxCluster + 1] = {};
+  int dev = 0;
+  NW_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return fail(NW_ERR_UNSUPPORTED, "device index above 63");
+  std::lock_guard<std::mutex> lock(mu);
+  if (slots[dev][size] == 0) {
+    auto k = nw::resident2d<float, 1, 2, false, false>;
+    const int smem = 200 * 1024;
+    NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem - 128));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = size;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    NW_CUDA(cudaOccupancyMaxActiveClusters(&n, k, &cfg));
+    slots[dev][size] = n > 0 ? n : -1;
+  }
+  *out = std::max(0, slots[dev][size]);
+  return NW_OK;
+}
+
+constexpr int kResidentSteps = 3;  // fewest forward steps worth loading the state for
+constexpr int kPmlRows = 6;  // at most, with a PML (registers)
+constexpr int kResidentRows[] = {2, 4, 6, 8, 12};  // rows per thread the resident kernels are built for
+
+// How a resident sweep covers the device (see resident2d.cuh).
+struct ResidentPlan {
+  bool ok = false;
+  int cluster = 0, strips = 0, rx = 0, nv = 0, threads = 0, max_rows = 0, cap_list = 0, cap_ent = 0;
+  int edge_lo = 0, edge_hi = 0, x0 = 0, x1 = 0;
+  bool pml = false;
+  size_t smem = 0;
+  double cost = 0.0;
+};
+
+template <typename T, int R, bool ADJ>
+int resident_plan(const nw_grid* g, const nw_medium* m, int n_shots, int n_rec, int n_cells, bool crowded,
+                  ResidentPlan* best) {
+  using L = nw::ResidentSmem<T, R>;
+  *best = ResidentPlan();
+  const bool pml = g->absorbing == NW_ABS_PML;
+  const int levels = pml && ADJ ? 3 : 2;
+  const int n0 = g->n[0], nv = (g->n[1] + L::VZ - 1) / L::VZ;
+  const int x0 = pml ? m->pml_core[0] : g->core_lo[0], x1 = pml ? m->pml_core[1] : g->core_hi[0];
+  const int z0 = pml ? m->pml_core[2] : g->core_lo[1], z1 = pml ? m->pml_core[3] : g->core_hi[1];
+  if (x0 < 0 || z0 < 0 || x1 < x0 || z1 < z0 || x1 > n0 || z1 > g->n[1]) return fail(NW_ERR_ARG, "medium.pml_core lies outside the grid");
+  int edge_lo = (z0 + L::VZ - 1) / L::VZ, edge_hi = z1 / L::VZ;
+  if (edge_lo >= edge_hi) edge_lo = edge_hi = nv;
+  const int ne = edge_lo + nv - edge_hi;
+  auto coef_per_row = [&](int rows) {
+    return pml ? L::pml_bytes(ne, nv, rows) : g->absorbing == NW_ABS_NONE ? (size_t)0 : L::coef_bytes(ne, rows);
+  };
+  for (int nc = 1; nc <= nw::kMaxCluster; ++nc) {
+    const int max_rows = (n0 + nc - 1) / nc, min_rows = n0 / nc;
+    if (min_rows < R || L::tables(nv, max_rows, levels) > kMaxSmem) continue;
+    int slots = 0;
+    const int rc = cluster_slots(nc, &slots);
+    if (rc) return rc;
+    if (slots < 1) continue;
+    for (int rx : kResidentRows) {
+      if (pml && rx > kPmlRows) continue;
+      for (int strips = (max_rows + rx - 1) / rx; strips <= min_rows / R && (strips - 1) * rx < 2 * max_rows; ++strips) {  // of R rows or more
+      // one service warp for every 64 receivers (touched cells) of an evenly loaded slab, up to four
+      const int serve = std::max(1, std::min(4, (ADJ ? n_cells : n_rec) / (64 * nc)));
+      const int cells = (strips * nv + 31) / 32 * 32;
+      const int threads = std::min(cells + 32 * serve, nw::resident_threads(pml));
+      if (threads < cells + 32) continue;
+      const size_t base = L::tables(nv, max_rows, levels) + (ADJ ? L::map_bytes(nv, max_rows) : 0) + coef_per_row(max_rows);
+      if (base > kMaxSmem) continue;
+      // the shared tables hold every receiver or touched cell, should all lie in one slab
+      const int cap_list = (ADJ ? n_cells : n_rec) / 4 * 4 + 4, cap_ent = ADJ ? 4 * n_rec + 4 : 0;
+      const size_t smem = base + cap_list * (ADJ ? L::cell_entry : L::list_entry) + cap_ent * L::csr_entry;
+      if (smem > kMaxSmem - 128 || (ADJ && n_cells > 4095)) continue;  // (12 bits of a vector's table entry)
+      // Cycles per step, from a sweep over grids of 117^2 to 552^2: a warp's row costs its shared-memory
+      // wavefronts (no other warp's overlaps them), a thread's rows run one after the other, and a step has
+      // its barriers and the halo's way to the neighbour. The adjoint's tallest strips, and a PML's, spill.
+      const int nr = (max_rows + strips - 1) / strips;
+      const double row = pml ? (ADJ ? (rx <= 4 ? 150.0 : 240.0) : 90.0) : ADJ ? (rx <= 8 ? 72.0 : 84.0) : 52.0;
+      const double chain = nr * (pml ? 750.0 : 250.0);
+      const double step = std::max(cells / 32 * nr * row, chain) + (nc > 1 ? 900.0 : 400.0);
+      // beside other sweeps that fill the device, what counts is the SMs' time
+      const double rounds = crowded ? (double)n_shots / slots : std::ceil((double)n_shots / slots);
+      const double cost = rounds * step;
+      if (!best->ok || cost < best->cost) {
+        best->ok = true;
+        best->cluster = nc; best->strips = strips; best->rx = rx; best->nv = nv; best->threads = threads;
+        best->max_rows = max_rows; best->edge_lo = edge_lo; best->edge_hi = edge_hi; best->x0 = x0; best->x1 = x1; best->pml = pml; best->cap_list = cap_list; best->cap_ent = cap_ent; best->smem = smem;
+        best->cost = cost;
+      }
+      }
+    }
+  }
+  return NW_OK;
+}
+
+template <typename T, int R, int RX, bool ADJ, bool PML>
+int launch_resident_r(const nw::KGrid<T>& kg, const nw::Resident<T>& a, const ResidentPlan& p, int n_shots,
+                      cudaStream_t s) {
+  auto k = nw::resident2d<T, R, RX, ADJ, PML>;
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  NW_CUDA(cudaGetDevice(&dev));
+  if (!done[dev & 63].load()) {
+    NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem - 128));
+    done[dev & 63].store(true);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.cluster * n_shots));
+  cfg.blockDim = dim3(p.threads);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = p.cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  NW_CUDA(cudaLaunchKernelEx(&cfg, k, kg, a));
+  NW_LAUNCHED();
+  return NW_OK;
+}
+
+template <typename T, int R, bool ADJ>
+int launch_resident_v(const nw::KGrid<T>& kg, const nw::Resident<T>& a, const ResidentPlan& p, int n_shots,
+                      cudaStream_t s) {
+  if (p.pml) {
+    switch (p.rx) {
+      case 2: return launch_resident_r<T, R, 2, ADJ, true>(kg, a, p, n_shots, s);
+      case 4: return launch_resident_r<T, R, 4, ADJ, true>(kg, a, p, n_shots, s);
+      default: return launch_resident_r<T, R, 6, ADJ, true>(kg, a, p, n_shots, s);
+    }
+  }
+  switch (p.rx) {
+    case 2: return launch_resident_r<T, R, 2, ADJ, false>(kg, a, p, n_shots, s);
+    case 4: return launch_resident_r<T, R, 4, ADJ, false>(kg, a, p, n_shots, s);
+    case 6: return launch_resident_r<T, R, 6, ADJ, false>(kg, a, p, n_shots, s);
+    case 8: return launch_resident_r<T, R, 8, ADJ, false>(kg, a, p, n_shots, s);
+    default: return launch_resident_r<T, R, 12, ADJ, false>(kg, a, p, n_shots, s);
+  }
+}
+
+// The plan of a forward or adjoint resident sweep of these shots (ok = false: the grid does not fit a
+// cluster's shared memory and registers, or has three dimensions).
+template <typename T, bool ADJ>
+int resident_for(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t, ResidentPlan* p,
+                 bool crowded = false) {
+  *p = ResidentPlan();
+  if (g->ndim != 2) return NW_OK;
+  if ((long long)a->n_rec * t->n_t > INT_MAX) return NW_OK;
+  auto plan = [&](bool c) {
+    return g->radius == 1 ? resident_plan<T, 1, ADJ>(g, m, a->n_shots, a->n_rec, a->n_cells, c, p)
+                          : resident_plan<T, 2, ADJ>(g, m, a->n_shots, a->n_rec, a->n_cells, c, p);
+  };
+  int rc = plan(false);
+  if (rc || !p->ok) return rc;
+  // against one-step launches: cycles per step of the launch chain, or of the cells at the rate the tiled
+  // kernels step them (16 shots of 552^2: 16.3 us forward, 18.1 us adjoint; with a PML 23.9 and 29.7 us)
+  const double cells = (double)g->n[0] * g->n[1] * a->n_shots * sizeof(T) / 4;
+  const double tiled = p->pml ? (ADJ ? 13000.0 + cells / 110.0 : 12000.0 + cells / 140.0)
+                              : std::max(4800.0, 1500.0 + cells / (ADJ ? 145.0 : 160.0));
+  if (p->cost >= tiled) {
+    p->ok = false;
+    return NW_OK;
+  }
+  return crowded ? plan(true) : NW_OK;  // (the route is the one the problem takes alone)
+}
+
+template <typename T>
+nw::Resident<T> resident_args(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
+                              const ResidentPlan& p) {
+  nw::Resident<T> r = {};
+  r.C = (const T*)m->c2dt2;
+  r.A = (const T*)m->coef_a;
+  r.B = (const T*)m->coef_b;
+  r.cluster = p.cluster;
+  r.nv = p.nv;
+  r.strips = p.strips;
+  r.max_rows = p.max_rows;
+  r.edge_lo = p.edge_lo;
+  r.edge_hi = p.edge_hi;
+  r.core_x0 = p.x0;
+  r.core_x1 = p.x1;
+  if (p.pml) {
+    r.zz = (const T*)m->pml_zz;
+    for (int ax = 0; ax < 2; ++ax) {
+      r.alpha[ax] = (const T*)m->pml_alpha[ax];
+      r.beta[ax] = (const T*)m->pml_beta[ax];
+    }
+    r.hx2 = (T)m->pml_half_inv_h[0];
+    r.hz2 = (T)m->pml_half_inv_h[1];
+  }
+  for (int i = 0; i <= p.cluster; ++i) r.slab[i] = (int)((long long)g->n[0] * i / p.cluster);
+  r.wc = nw::lane_weight((T)g->w_center);
+  r.w1x = nw::lane_weight((T)g->w1[0]);
+  r.w1z = nw::lane_weight((T)g->w1[1]);
+  r.w2x = nw::lane_weight((T)g->w2[0]);
+  r.w2z = nw::lane_weight((T)g->w2[1]);
+  r.minus_one = nw::lane_weight(T(-1));
+  r.substeps = t->substeps;
+  r.first_b_one = t->first_b_one;
+  r.level = (long long)a->n_shots * g->field_elems;
+  r.n_rec = a->n_rec;
+  r.n_t = t->n_t;
+  r.n_cells = a->n_cells;
+  r.cap_list = p.cap_list;
+  r.cap_ent = p.cap_ent;
+  return r;
+}
+
+// Forward steps [n, n_end) of all shots in one launch: levels L(n-1), L(n) -> L(n_end-1), L(n_end); Lap p of
+// step n into lap (consecutive levels) when given.
+template <typename T>
+int resident_forward(const nw_grid* g, const nw::KGrid<T>& kg, const nw_medium* m, const nw_acquisition* a,
+                     const nw_time* t, const ResidentPlan& p, T* prev, T* cur, T* out_prev, T* out_cur, int n,
+                     int n_end, T* traces, T* lap, T* psi, cudaStream_t s, const T* const* faces = nullptr,
+                     const nw_storage* snaps = nullptr) {
+  nw::Resident<T> r = resident_args<T>(g, m, a, t, p);
+  if (p.pml)
+    for (int ax = 0; ax < 2; ++ax) {  // psi levels 2 * axis + step parity, or the given ones of step n
+      r.f_in[ax] = faces ? faces[ax] : psi + (long long)(2 * ax + n % 2) * r.level;
+      r.f_out[ax] = psi + (long long)(2 * ax + n_end % 2) * r.level;
+    }
+  if (snaps) {
+    r.snap = (T*)snaps->snap;
+    r.segment = snaps->segment;
+    r.snap_stride = (long long)(snap_layout(g, a->n_shots).per_snap(NW_SNAP_EXACT) / sizeof(T));
+  }
+  r.in_prev = prev;
+  r.in_cur = cur;
+  r.out_prev = out_prev;
+  r.out_cur = out_cur;
+  r.n_first = n;
+  r.count = n_end - n;
+  r.src_corner = a->has_source ? a->src_corner : nullptr;
+  r.src_w = (const T*)a->src_weight;
+  r.wavelet = (const T*)a->wavelet;
+  r.traces = a->n_rec > 0 ? traces : nullptr;
+  r.rec_corner = a->rec_corner;
+  r.rec_w = (const T*)a->rec_weight;
+  r.lap_out = lap;
+  return g->radius == 1 ? launch_resident_v<T, 1, false>(kg, r, p, a->n_shots, s)
+                        : launch_resident_v<T, 2, false>(kg, r, p, a->n_shots, s);
+}
+
+// Adjoint steps n, n-1, ..., n_last of all shots in one launch: levels q^{n+2}, q^{n+1} in (prev, cur) become
+// q^{n_last+1}, q^{n_last} in place; acc holds one gradient sum per shot; lap points at Lap p of step lap_n0,
+// steps [lap_n0, lap_end) have one.
+template <typename T>
+int resident_adjoint(const nw_grid* g, const nw::KGrid<T>& kg, const nw_medium* m, const nw_acquisition* a,
+                     const nw_time* t, const ResidentPlan& p, T* prev, T* cur, T* acc, int n, int n_last,
+                     const T* gtr, const T* lap, int lap_n0, int lap_end, T* faces, cudaStream_t s) {
+  nw::Resident<T> r = resident_args<T>(g, m, a, t, p);
+  if (p.pml)
+    for (int ax = 0; ax < 2; ++ax) {  // step n reads parity n + 1 and writes parity n
+      r.f_in[ax] = faces + (long long)(2 * ax + (n + 1) % 2) * r.level;
+      r.f_out[ax] = faces + (long long)(2 * ax + n_last % 2) * r.level;
+    }
+  r.in_prev = r.out_prev = prev;
+  r.in_cur = r.out_cur = cur;
+  r.n_first = n;
+  r.count = n - n_last + 1;
+  r.gtr = a->n_cells > 0 ? gtr : nullptr;
+  r.cell_index = a->cell_index;
+  r.cell_ptr = a->cell_ptr;
+  r.cell_rec = a->cell_rec;
+  r.cell_w = (const T*)a->cell_weight;
+  r.lap = lap;
+  r.lap_n0 = lap_n0;
+  r.lap_end = lap_end;
+  r.acc = acc;
+  return g->radius == 1 ? launch_resident_v<T, 1, true>(kg, r, p, a->n_shots, s)
+                        : launch_resident_v<T, 2, true>(kg, r, p, a->n_shots, s);
+}
+
 // ---- forward driver ---------------------------------------------------------------------
 // The PML coefficients of a medium into a step descriptor.
 template <typename T>
@@ -544,6 +832,59 @@ int fork_join(cudaStream_t s, bool with_side, FS side, FM main) {
   const cudaError_t ew = ej == cudaSuccess ? cudaStreamWaitEvent(s, ss->join, 0) : ej;
   if (rc) return rc;
   if (ew != cudaSuccess) return fail(NW_ERR_CUDA, std::string("side stream join: ") + cudaGetErrorString(ew));
+  return NW_OK;
+}
+
+// Streams of the calling thread on the current device for sweeps that do not depend on each other, forked
+// from a caller's stream and joined back into it (bounded, created at first use, kept until the process
+// exits, like the side stream).
+constexpr int kLanes = 8;
+struct Lanes {
+  cudaStream_t s[kLanes] = {};
+  cudaEvent_t fork = nullptr, join[kLanes] = {};
+};
+int lanes(Lanes** out) {
+  thread_local Lanes per_device[64];
+  int dev = 0;
+  NW_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return fail(NW_ERR_UNSUPPORTED, "device index above 63");
+  Lanes& r = per_device[dev];
+  if (!r.fork) {  // in relaxed capture mode, as the side stream
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    NW_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < kLanes && !e; ++i) {
+      if (!r.s[i]) e = cudaStreamCreateWithFlags(&r.s[i], cudaStreamNonBlocking);
+      if (!e && !r.join[i]) e = cudaEventCreateWithFlags(&r.join[i], cudaEventDisableTiming);
+    }
+    if (!e) e = cudaEventCreateWithFlags(&r.fork, cudaEventDisableTiming);
+    NW_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    if (e != cudaSuccess) return fail(NW_ERR_CUDA, std::string("lane streams: ") + cudaGetErrorString(e));
+  }
+  *out = &r;
+  return NW_OK;
+}
+
+// work(lane streams) between a fork from s and a join back into it of the first n lanes; joined on every
+// path, errors included, so that a capture of s never ends with one still forked.
+template <typename F>
+int on_lanes(cudaStream_t s, int n, F work) {
+  if (n <= 0) return NW_OK;
+  Lanes* l = nullptr;
+  int rc = lanes(&l);
+  if (rc) return rc;
+  NW_CUDA(cudaEventRecord(l->fork, s));
+  cudaError_t e = cudaSuccess;
+  int forked = 0;
+  while (forked < n && (e = cudaStreamWaitEvent(l->s[forked], l->fork, 0)) == cudaSuccess) ++forked;
+  if (e == cudaSuccess) rc = work(l->s);
+  for (int i = 0; i < forked; ++i) {
+    cudaError_t j = cudaEventRecord(l->join[i], l->s[i]);
+    if (j == cudaSuccess) j = cudaStreamWaitEvent(s, l->join[i], 0);
+    if (e == cudaSuccess) e = j;
+  }
+  if (rc) return rc;
+  if (e != cudaSuccess) return fail(NW_ERR_CUDA, std::string("lane streams: ") + cudaGetErrorString(e));
   return NW_OK;
 }
 
@@ -760,7 +1101,8 @@ int forward_step(const nw_grid* g, const nw::KGrid<T>& kg, const nw_medium* m, c
 
 template <typename T>
 int forward_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
-                 const nw_storage* st, const Tune& tu, int n_begin, int n_end, T* traces, cudaStream_t s) {
+                 const nw_storage* st, const Tune& tu, int n_begin, int n_end, T* traces, cudaStream_t s,
+                 bool crowded = false) {
   const long long LE = (long long)a->n_shots * g->field_elems;
   if (!st->ring) return fail(NW_ERR_ARG, "storage needs a ring buffer");
   Ring<T> L;
@@ -777,8 +1119,20 @@ int forward_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
     return !(ckpt && n % st->segment == 0) ? -1 : st->snap_slot ? st->snap_slot[n / st->segment] : n / st->segment;
   };
   const bool pairs = g->ndim == 2 && tu.fwd.depth == 2 && L.levels == 4;
+  ResidentPlan res;
+  if (!pairs) {
+    const int rc = resident_for<T, false>(g, m, a, t, &res, crowded);
+    if (rc) return rc;
+  }
+  // a resident sweep writes exact snapshots itself (their ghost cells stay zero)
+  const bool own_snaps = res.ok && ckpt && !st->snap_slot && st->snap_kind == NW_SNAP_EXACT && n_end - n_begin >= kResidentSteps;
+  if (own_snaps) {
+    const size_t per = snap_layout(g, a->n_shots).per_snap(NW_SNAP_EXACT);
+    const int j0 = (n_begin + st->segment - 1) / st->segment, j1 = (n_end + st->segment - 1) / st->segment;
+    if (j1 > j0) NW_CUDA(cudaMemsetAsync((char*)st->snap + (size_t)j0 * per, 0, (size_t)(j1 - j0) * per, s));
+  }
   for (int n = n_begin; n < n_end;) {
-    const int slot = slot_at(n);
+    const int slot = own_snaps ? -1 : slot_at(n);
     if (slot >= 0) {
       T* faces[2];
       if (pml) pml_faces<T>((T*)st->pml_psi, LE, n, faces);
@@ -786,6 +1140,17 @@ int forward_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
       if (rc) return rc;
     }
     T* lap = st->history ? (T*)st->history + (long long)n * LE : nullptr;
+    if (res.ok) {  // up to the next snapshot in one launch (one or two steps go through the one-step kernel)
+      int next = n + 1;
+      while (next < n_end && (own_snaps || slot_at(next) < 0)) ++next;
+      if (next - n >= kResidentSteps) {
+        const int rc = resident_forward<T>(g, kg, m, a, t, res, L.at(n - 1), L.at(n), L.at(next - 1), L.at(next), n,
+                                           next, traces, lap, (T*)st->pml_psi, s, nullptr, own_snaps ? st : nullptr);
+        if (rc) return rc;
+        n = next;
+        continue;
+      }
+    }
     if (pairs && n + 1 < n_end && slot_at(n + 1) < 0) {  // steps n and n+1 in one launch
       int rc = forward_pair<T>(g, kg, m, a, t, tu, L, n, true, traces, lap, lap ? lap + LE : nullptr, s);
       if (rc) return rc;
@@ -813,7 +1178,7 @@ int grid_blocks(long long work, int threads) {
 template <typename T>
 int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
                  const nw_storage* st, const Tune& tu, const T* gtr, T* work, T* gacc, T* lambda0,
-                 T* mu1, cudaStream_t s) {
+                 T* mu1, cudaStream_t s, bool crowded = false) {
   const int N = t->n_steps, M = t->substeps, S = a->n_shots;
   const long long LE = (long long)S * g->field_elems;
   const size_t lvl_bytes = (size_t)LE * sizeof(T);
@@ -833,8 +1198,17 @@ int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
   L.level_elems = LE;
   L.levels = ckpt ? ring_levels(st) : 3;
   const bool pairs = g->ndim == 2 && tu.fwd.depth == 2 && L.levels == 4;
+  ResidentPlan res, fres;  // the adjoint's and the recompute's resident sweeps
+  {
+    int rc = resident_for<T, true>(g, m, a, t, &res, crowded);
+    if (!rc && ckpt && !pairs) rc = resident_for<T, false>(g, m, a, t, &fres, crowded);
+    if (rc) return rc;
+  }
   // forward steps [k0, k1) of a recompute or an advance; Lap p^k into seg + (k - k0) levels if seg
   auto recompute = [&](int k0, int k1, T* seg) -> int {
+    if (fres.ok && k1 - k0 >= kResidentSteps)
+      return resident_forward<T>(g, kg, m, a, t, fres, L.at(k0 - 1), L.at(k0), L.at(k1 - 1), L.at(k1), k0, k1, nullptr,
+                                 seg, (T*)st->pml_psi, s);
     for (int k = k0; k < k1;) {
       T* lp = seg ? seg + (long long)(k - k0) * LE : nullptr;
       if (pairs && k + 1 < k1) {
@@ -937,7 +1311,21 @@ int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
     }
     return box_inject ? NW_OK : inject3(n);  // (inject3 itself skips the steps without cotangents)
   };
-  if (N >= n_stop) {  // level N: q^N = A C R^T g_N (q^{N+1} = q^{N+2} = 0)
+  // A resident sweep keeps q^{n+1}, q^{n+2} in the first two work levels and one gradient sum per shot in
+  // the third; lv1, lv0 are q^1 and q^0 at the end.
+  T *lv0 = res.ok ? work : q(0), *lv1 = res.ok ? work + LE : q(1);
+  T* racc = res.pml ? gacc : work + 2 * LE;  // (with a PML the accumulators are per shot already)
+  if (res.ok) {
+    if (hist) {
+      const int rc = N >= n_stop ? resident_adjoint<T>(g, kg, m, a, t, res, work + LE, work, racc, N, n_stop, gtr,
+                                                       (const T*)st->history, 0, N, work + 3 * LE, s)
+                                 : NW_OK;
+      if (rc) return rc;
+    } else if (N >= n_stop) {
+      const int rc = resident_adjoint<T>(g, kg, m, a, t, res, work + LE, work, racc, N, N, gtr, nullptr, N, N, work + 3 * LE, s);
+      if (rc) return rc;
+    }
+  } else if (N >= n_stop) {  // level N: q^N = A C R^T g_N (q^{N+1} = q^{N+2} = 0)
     int rc = pml ? step_pml(N, nullptr) : (g->ndim == 2 ? step2(N, nullptr) : inject3(N));
     if (rc) return rc;
   }
@@ -976,7 +1364,7 @@ int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
     }
     return fail(NW_ERR_ARG, "schedule: ended before the YOUTURN of segment " + std::to_string(seg));
   };
-  for (int n = N - 1; n >= n_stop; --n) {
+  for (int n = res.ok && hist ? n_stop - 1 : N - 1; n >= n_stop; --n) {
     const T* lap;
     if (hist) {
       lap = (const T*)st->history + (long long)n * LE;
@@ -985,16 +1373,34 @@ int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
       if (seg_n0 != n0) {  // entering a segment from its end: recompute Lap p^{n0..n1-1}
         const int n1 = std::min(n0 + K, N);
         seg_n0 = n0;
+        bool recomputed = false;
         T* faces[2];  // with a PML the recompute runs its face fields in storage.pml_psi
         if (pml) pml_faces<T>((T*)st->pml_psi, LE, n0, faces);
+        if (fres.ok && !prog && st->snap_kind == NW_SNAP_EXACT && n1 - n0 >= kResidentSteps) {
+          // straight from the snapshot (p^{n0-1}, p^{n0}, the face fields), keeping only Lap p
+          T* snap = (T*)((char*)st->snap + (size_t)(n0 / K) * snap_layout(g, S).per_snap(NW_SNAP_EXACT));
+          const T* sf[2] = {snap + 2 * LE, snap + 3 * LE};
+          const int rc = resident_forward<T>(g, kg, m, a, t, fres, snap, snap + LE, nullptr, nullptr, n0, n1, nullptr,
+                                             (T*)st->segbuf, (T*)st->pml_psi, s, sf);
+          if (rc) return rc;
+          recomputed = true;
+        }
         // the ring to the segment's start: the schedule's program, or the segment's own snapshot
-        int rc = prog ? run_program(n0 / K)
+        int rc = recomputed ? NW_OK : prog ? run_program(n0 / K)
                       : snap_load<T>(g, st, S, n0 / K, L.at(n0 - 1), L.at(n0), s, pml ? faces : nullptr);
         if (rc) return rc;
-        rc = recompute(n0, n1, (T*)st->segbuf);
+        if (!recomputed) rc = recompute(n0, n1, (T*)st->segbuf);
         if (rc) return rc;
       }
       lap = (const T*)st->segbuf + (long long)(n - n0) * LE;
+      if (res.ok) {  // the segment's steps in one launch
+        const int n_last = std::max(n0, n_stop);
+        const int rc = resident_adjoint<T>(g, kg, m, a, t, res, work + LE, work, racc, n, n_last, gtr,
+                                           (const T*)st->segbuf, n0, n + 1, work + 3 * LE, s);
+        if (rc) return rc;
+        n = n_last;
+        continue;
+      }
     }
     if (pml) {
       int rc = step_pml(n, lap);
@@ -1021,16 +1427,21 @@ int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
     rc = inject3(n);
     if (rc) return rc;
   }
+  if (res.ok && !res.pml && N > 0) {  // the accumulator fields: the shots of a group summed in order
+    const dim3 gg(grid_blocks(g->field_elems, 256), tu.adj.groups(S));
+    nw::group_sum_kernel<T><<<gg, 256, 0, s>>>(work + 2 * LE, g->field_elems, S, tu.adj.spc, gacc);
+    NW_LAUNCHED();
+  }
   if (lambda0) {  // lambda^0 = q^0 / C and mu^1 = q^1 / C on the padded grid, zero ghosts
     NW_CUDA(cudaMemsetAsync(lambda0, 0, lvl_bytes, s));
     const long long cells = (long long)g->n[0] * g->n[1] * (g->ndim == 3 ? g->n[2] : 1);
     dim3 ug(grid_blocks(cells, 256), S);
-    nw::unscale_kernel<T><<<ug, 256, 0, s>>>(kg, g->ndim, (const T*)m->c2dt2, q(0), lambda0);
+    nw::unscale_kernel<T><<<ug, 256, 0, s>>>(kg, g->ndim, (const T*)m->c2dt2, lv0, lambda0);
     NW_LAUNCHED();
     if (mu1) {
       NW_CUDA(cudaMemsetAsync(mu1, 0, lvl_bytes, s));
       if (N > 0) {
-        nw::unscale_kernel<T><<<ug, 256, 0, s>>>(kg, g->ndim, (const T*)m->c2dt2, q(1), mu1);
+        nw::unscale_kernel<T><<<ug, 256, 0, s>>>(kg, g->ndim, (const T*)m->c2dt2, lv1, mu1);
         NW_LAUNCHED();
       }
     }
@@ -1332,7 +1743,8 @@ int nw_status(void* stream) {
   if (v) {
     const int zero = 0;
     NW_CUDA(cudaMemcpyToSymbol(nw::g_status, &zero, sizeof(int)));
-    return fail(v, "a snapshot block held a non-finite value or scale");
+    return fail(v, v == NW_ERR_TIMEOUT ? "a wait for a neighbouring CTA's rows gave up"
+                                       : "a snapshot block held a non-finite value or scale");
   }
   return NW_OK;
 }
@@ -1470,7 +1882,17 @@ int check_batch(const nw_batch_problem* P, int n, const Tune& tu) {
 // (the layer goes through the PML kernel in launches of its own). The box depends on T only through
 // its 16-byte column alignment, which the batch's dtype fixes.
 template <typename T>
+int batch_solo(const nw_batch_problem& q, bool* solo) {  // whether q takes resident sweeps: it then runs apart
+  ResidentPlan f, a;
+  int rc = resident_for<T, false>(&q.grid, &q.medium, &q.acq, &q.time, &f);
+  if (!rc) rc = resident_for<T, true>(&q.grid, &q.medium, &q.acq, &q.time, &a);
+  *solo = f.ok || a.ok;
+  return rc;
+}
+template <typename T>
 dim3 batch_grid(const nw_batch_problem& q, const TileCfg& c) {
+  bool solo = false;
+  if (batch_solo<T>(q, &solo) || solo) return dim3(0, 0, 0);
   if (q.grid.absorbing != NW_ABS_PML) return c.grid(&q.grid, q.acq.n_shots);
   nw::PmlStep<T> st = {};
   if (pml_tiled_box<T>(&q.grid, &q.medium, c, st) || st.kx1 == st.kx0) return dim3(0, 0, 0);
@@ -1556,6 +1978,40 @@ int batch_prepare_impl(const nw_batch_problem* P, int n, const Tune& tu, void* t
   acta[n] = (int)asum;
   NW_CUDA(cudaMemcpyAsync(table, host.data(), L.bytes, cudaMemcpyHostToDevice, s));
   NW_CUDA(cudaStreamSynchronize(s));  // the host staging copy dies with this call
+  return NW_OK;
+}
+
+// The problems whose sweeps are resident, shared over the lanes (the costliest first, each to the least
+// loaded lane): run(problem, lane stream) for each, beside rest() on s.
+template <typename F, typename G>
+int batch_solos(const nw_batch_problem* P, const std::vector<char>& solo, cudaStream_t s, F run, G rest) {
+  std::vector<int> order;
+  for (int p = 0; p < (int)solo.size(); ++p)
+    if (solo[p]) order.push_back(p);
+  auto cost = [&](int p) { return (double)P[p].grid.field_elems * P[p].acq.n_shots * P[p].time.n_steps; };
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
+  const int n = std::min((int)order.size(), kLanes);
+  if (n == 0) return rest();
+  return on_lanes(s, n, [&](cudaStream_t* lane) -> int {
+    double load[kLanes] = {};
+    for (int p : order) {
+      const int l = (int)(std::min_element(load, load + n) - load);
+      load[l] += cost(p);
+      const int rc = run(P[p], lane[l]);
+      if (rc) return rc;
+    }
+    return rest();
+  });
+}
+template <typename T>
+int batch_solo_flags(const nw_batch_problem* P, int n, std::vector<char>* solo) {
+  solo->assign(n, 0);
+  for (int p = 0; p < n; ++p) {
+    bool f = false;
+    const int rc = batch_solo<T>(P[p], &f);
+    if (rc) return rc;
+    (*solo)[p] = f;
+  }
   return NW_OK;
 }
 
@@ -1723,10 +2179,16 @@ int batch_forward_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
     NW_CUDA(cudaMemsetAsync(P[p].storage.ring, 0, 3 * lvl, s));
     if (P[p].grid.absorbing == NW_ABS_PML) NW_CUDA(cudaMemsetAsync(P[p].storage.pml_psi, 0, 4 * lvl, s));
   }
+  std::vector<char> solo;
+  int rc0 = batch_solo_flags<T>(P, n, &solo);
+  if (rc0) return rc0;
+  auto tiled_pml = [&](int p) { return P[p].grid.absorbing == NW_ABS_PML && !solo[p]; };
+  auto rest = [&]() -> int {  // the others, together, a step per launch
   for (int k = 0; k < Nmax; ++k) {
     const int na = batch_active(P, n, k, false);
     if (k % K == 0)
       for (int p = 0; p < na; ++p) {
+        if (solo[p]) continue;
         const bool pml = P[p].grid.absorbing == NW_ABS_PML;
         T* faces[2];
         if (pml) batch_pml_faces<T>(P[p], k, faces);
@@ -1735,13 +2197,13 @@ int batch_forward_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
         if (rc) return rc;
       }
     bool any_pml = false;
-    for (int p = 0; p < na; ++p) any_pml |= P[p].grid.absorbing == NW_ABS_PML;
+    for (int p = 0; p < na; ++p) any_pml |= tiled_pml(p);
     int rc = fork_join(
         s, any_pml,
         [&](cudaStream_t t) -> int {  // PML problems: receivers of level k and the layer cells
           for (int p = 0; p < na; ++p) {
             const nw_batch_problem& q = P[p];
-            if (q.grid.absorbing != NW_ABS_PML) continue;
+            if (!tiled_pml(p)) continue;
             int r = NW_OK;
             if (k % q.time.substeps == 0)
               r = launch_sample<T>(&q.grid, &q.acq, q.time.n_t, ring_level<T>(q, k), k / q.time.substeps,
@@ -1755,7 +2217,7 @@ int batch_forward_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
     if (rc) return rc;
     for (int p = 0; p < na; ++p) {  // the final receiver sample of problems ending after step k
       const nw_batch_problem& q = P[p];
-      if (q.time.n_steps == k + 1 && q.time.n_steps % q.time.substeps == 0) {
+      if (!solo[p] && q.time.n_steps == k + 1 && q.time.n_steps % q.time.substeps == 0) {
         rc = launch_sample<T>(&q.grid, &q.acq, q.time.n_t, ring_level<T>(q, k + 1), (k + 1) / q.time.substeps,
                               (T*)q.traces, s);
         if (rc) return rc;
@@ -1763,13 +2225,25 @@ int batch_forward_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
     }
   }
   return NW_OK;
+  };
+  return batch_solos(P, solo, s,
+                     [&](const nw_batch_problem& q, cudaStream_t lane) {
+                       return forward_impl<T>(&q.grid, &q.medium, &q.acq, &q.time, &q.storage, tu, 0, q.time.n_steps,
+                                              (T*)q.traces, lane, true);
+                     },
+                     rest);
 }
 
 template <typename T>
 int batch_adjoint_impl(const nw_batch_problem* P, int n, const Tune& tu, const void* table, cudaStream_t s) {
   const int K = P[0].storage.segment, Nmax = P[0].time.n_steps, R = P[0].grid.radius;
   const std::vector<int> fcta = batch_ctas<T>(P, n, tu.fwd), acta = batch_ctas<T>(P, n, tu.adj);
+  std::vector<char> solo;
+  int rc0 = batch_solo_flags<T>(P, n, &solo);
+  if (rc0) return rc0;
+  auto tiled_pml = [&](int p) { return P[p].grid.absorbing == NW_ABS_PML && !solo[p]; };
   for (int p = 0; p < n; ++p) {
+    if (solo[p]) continue;
     const nw_batch_problem& q = P[p];
     const size_t lvl = (size_t)q.acq.n_shots * q.grid.field_elems * sizeof(T);
     NW_CUDA(cudaMemsetAsync(q.work, 0, work_levels(&q.grid) * lvl, s));
@@ -1778,12 +2252,12 @@ int batch_adjoint_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
   auto adj_step = [&](int step) -> int {
     const int na = batch_active(P, n, step, true);
     bool any_pml = false;
-    for (int p = 0; p < na; ++p) any_pml |= P[p].grid.absorbing == NW_ABS_PML;
+    for (int p = 0; p < na; ++p) any_pml |= tiled_pml(p);
     int rc = fork_join(
         s, any_pml,
         [&](cudaStream_t t) -> int {  // PML problems: the layer cells
           for (int p = 0; p < na; ++p)
-            if (P[p].grid.absorbing == NW_ABS_PML) {
+            if (tiled_pml(p)) {
               const int r = batch_pml_adjoint<T>(P[p], tu, step, t);
               if (r) return r;
             }
@@ -1791,15 +2265,17 @@ int batch_adjoint_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
         },
         [&](cudaStream_t t) -> int { return NW_DISPATCH_BATCH(launch_adj_batch, T, tu.adj, R, table, n, na, acta[na], step, 0, K, t); });
     for (int p = 0; p < na && !rc; ++p)  // and their cotangents, once both halves are done
-      if (P[p].grid.absorbing == NW_ABS_PML) rc = batch_pml_inject<T>(P[p], tu, step, s);
+      if (tiled_pml(p)) rc = batch_pml_inject<T>(P[p], tu, step, s);
     return rc;
   };
+  auto rest = [&]() -> int {
   int rc = adj_step(Nmax);  // problems with the largest step count start: q^N = A C R^T g_N
   if (rc) return rc;
   for (int seg = Nmax > 0 ? (Nmax - 1) / K : -1; seg >= 0; --seg) {
     const int n0 = seg * K, n1 = std::min(n0 + K, Nmax);
     const int na0 = batch_active(P, n, n0, false);
     for (int p = 0; p < na0; ++p) {  // decode the segment's snapshots into the rings (and faces)
+      if (solo[p]) continue;
       const bool pml = P[p].grid.absorbing == NW_ABS_PML;
       T* faces[2];
       if (pml) batch_pml_faces<T>(P[p], n0, faces);
@@ -1810,12 +2286,12 @@ int batch_adjoint_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
     for (int k = n0; k < n1; ++k) {  // recompute Lap p^k into the segment buffers
       const int na = batch_active(P, n, k, false);
       bool any_pml = false;
-      for (int p = 0; p < na; ++p) any_pml |= P[p].grid.absorbing == NW_ABS_PML;
+      for (int p = 0; p < na; ++p) any_pml |= tiled_pml(p);
       rc = fork_join(
           s, any_pml,
           [&](cudaStream_t t) -> int {
             for (int p = 0; p < na; ++p)
-              if (P[p].grid.absorbing == NW_ABS_PML) {
+              if (tiled_pml(p)) {
                 const int r = batch_pml_forward<T>(P[p], tu, k, true, t);
                 if (r) return r;
               }
@@ -1830,6 +2306,13 @@ int batch_adjoint_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
     }
   }
   return NW_OK;
+  };
+  return batch_solos(P, solo, s,
+                     [&](const nw_batch_problem& q, cudaStream_t lane) {
+                       return adjoint_impl<T>(&q.grid, &q.medium, &q.acq, &q.time, &q.storage, tu, (const T*)q.grad_traces,
+                                              (T*)q.work, (T*)q.grad_acc, (T*)nullptr, (T*)nullptr, lane, true);
+                     },
+                     rest);
 }
 
 }  // namespace
