@@ -92,6 +92,11 @@ struct Resident {
   const T* __restrict__ lap;  // Lap p of step 0 in memory order (step n at + (n - lap_n0) levels)
   int lap_n0, lap_end;        // steps [lap_n0, lap_end) have a Lap p; others add nothing to the gradient
   T* acc;                     // per-shot sums of q^{n+1} Lap p^n (read, added to, written)
+  // forward of a time reversal: after step n the imposed cells (field offsets, n_imposed) hold their traces at
+  // reversed time T - (n + 1) dt, linear between samples
+  const int64_t* __restrict__ imposed;
+  const T* __restrict__ imposed_tr;
+  int n_imposed;
   int n_rec, n_t, n_cells;
   int cap_list;  // receivers (forward) or touched cells (adjoint) the shared tables hold: at least all of them
   int cap_ent;   // adjoint: the table entries they hold
@@ -115,6 +120,8 @@ struct ResidentSmem {
   static constexpr size_t list_entry = 8 + 4 * sizeof(T);                 // forward: id, offset, 4 weights
   static constexpr size_t cell_entry = 4 + 2 * sizeof(T);                 // adjoint: first entry, 2 values
   static constexpr size_t csr_entry = 4 + sizeof(T);                      // offset, weight
+  static constexpr size_t imposed_entry = 4 + 2 * sizeof(T);              // trace, 2 values
+  __host__ __device__ static size_t lane_bytes(int nv, int rows) { return ((size_t)nv * rows * VZ * 2 + 15) / 16 * 16; }
   __host__ __device__ static size_t map_bytes(int nv, int rows) { return ((size_t)nv * rows * 2 + 15) / 16 * 16; }
   // A, B: one vector each per row (its columns between the layers, all alike), those of the edge vectors
   __host__ __device__ static size_t coef_bytes(int ne, int rows) { return (size_t)rows * (ne + 1) * 32; }
@@ -497,7 +504,37 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
   int* e_off = c_first + a.cap_list;                         // [cap_ent] receiver * n_t
   // count[0], count[1]: receivers inside the slab, and those that also read the halo below (at the list's
   // end); touched cells and entries
+  unsigned short* lane_map = reinterpret_cast<unsigned short*>(tables);  // time reversal: a cell's entry + 1
+  T* i_val = reinterpret_cast<T*>(tables + L::lane_bytes(a.nv, a.max_rows));  // [2][n_imposed] values by step parity
+  int* i_row = reinterpret_cast<int*>(i_val + 2 * a.n_imposed);               // trace row
+  auto imposed_values = [&](int n, T* dst, int id, int step) {  // of level n
+    const double u = (a.n_t - 1) - (double)n / a.substeps;
+    const int j0 = min(max((int)floor(u), 0), a.n_t - 1), j1 = min(j0 + 1, a.n_t - 1);
+    const double w = u - j0;
+    for (int e = id, n_in = count[0]; e < n_in; e += step) {
+      const T* tr = a.imposed_tr + (long long)i_row[e] * a.n_t;
+      dst[e] = add_rn(mul_rn((T)(1.0 - w), tr[j0]), mul_rn((T)w, tr[j1]));
+    }
+  };
   if constexpr (!ADJ) {
+    if (a.imposed) {
+      for (int i = tid; i < a.nv * rows * VZ; i += nthr) lane_map[i] = 0;
+      __syncthreads();
+      for (int c = tid; c < a.n_imposed; c += nthr) {
+        const int rel = (int)(a.imposed[c] - g.origin) - X0 * ld;
+        if (rel < 0 || rel >= rows * ld) continue;
+        const int e = atomicAdd(count, 1), r = rel / ld;
+        i_row[e] = c;
+        lane_map[r * a.nv * VZ + rel - r * ld] = (unsigned short)(e + 1);
+      }
+      __syncthreads();
+      imposed_values(a.n_first + 1, i_val, tid, nthr);
+      if (work)
+        for (int k = 0; k < nr; ++k)
+#pragma unroll
+          for (int v = 0; v < VZ; ++v)
+            if (lane_map[(r0 + dir * k) * a.nv * VZ + zc + v]) rare |= 1u << k;
+    }
     if (a.traces) {
       if (tid == 0) count[1] = 0;
       __syncthreads();
@@ -746,7 +783,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
         }
         v_fma(cc[C_REG ? k : k % PF], lp, two, o);
         if constexpr (!ADJ) {
-          if (now >> k & 1u) {  // the source
+          if (a.src_corner && (now >> k & 1u)) {  // the source
             const int dx = r0 + dir * k + X0 - a.src_corner[2 * s], z0 = zc - a.src_corner[2 * s + 1];
             const T* w = src_sh + 4 * (m & 1) + 2 * dx;
 #pragma unroll
@@ -755,6 +792,15 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
           }
         }
         if constexpr (LAYER) v_mul(ca, o, o);
+        if constexpr (!ADJ) {
+          if (a.imposed && (now >> k & 1u)) {
+#pragma unroll
+            for (int v = 0; v < VZ; ++v) {
+              const int e = lane_map[(r0 + dir * k) * a.nv * VZ + zc + v];
+              if (e) o[v] = i_val[(m & 1) * a.n_imposed + e - 1];
+            }
+          }
+        }
         vstore<T, VZ>(out, o);
         if constexpr (!ADJ) {
           if (lps) {  // (whole vectors: nothing reads the ghost columns of a stored Laplacian)
@@ -972,7 +1018,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
               lp[v] = add_rn(lp[v], px[v]);
               o[v] = fma_rn(-cZ[v], wv[R][v], fma_rn(cc[k][v], lp[v], fma_rn(-cB[v], pv[v], add_rn(wv[R][v], wv[R][v]))));
             }
-            if (now >> k & 1u) {  // the source
+            if (a.src_corner && (now >> k & 1u)) {  // the source
               const int dx = r0 + k + X0 - a.src_corner[2 * s], z0 = zc - a.src_corner[2 * s + 1];
               const T* wgt = src_sh + 4 * (m & 1) + 2 * dx;
 #pragma unroll
@@ -981,6 +1027,13 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
             }
 #pragma unroll
             for (int v = 0; v < VZ; ++v) o[v] = mul_rn(cA[v], o[v]);
+            if (a.imposed && (now >> k & 1u)) {
+#pragma unroll
+              for (int v = 0; v < VZ; ++v) {
+                const int e = lane_map[(r0 + k) * a.nv * VZ + zc + v];
+                if (e) o[v] = i_val[(m & 1) * a.n_imposed + e - 1];
+              }
+            }
             if (lps) {
               vstore<T, VZ>(lps, lp);
               lps += dl;
@@ -1088,6 +1141,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
           src_sh[4 * (1 - (m & 1)) + id] = mul_rn(weight, wave);
           if (m + 2 < a.count) wave = a.wavelet[n + 2];
         }
+        if (a.imposed && !last) imposed_values(n + 2, i_val + (1 - (m & 1)) * a.n_imposed, id, ns);
         if (++phase == a.substeps) { phase = 0; ++j; }
       }
       cta_barrier();

@@ -510,8 +510,8 @@ struct ResidentPlan {
 };
 
 template <typename T, int R, bool ADJ>
-int resident_plan(const nw_grid* g, const nw_medium* m, int n_shots, int n_rec, int n_cells, bool crowded,
-                  ResidentPlan* best) {
+int resident_plan(const nw_grid* g, const nw_medium* m, int n_shots, int n_rec, int n_cells, int n_imposed,
+                  bool crowded, ResidentPlan* best) {
   using L = nw::ResidentSmem<T, R>;
   *best = ResidentPlan();
   const bool pml = g->absorbing == NW_ABS_PML;
@@ -545,7 +545,9 @@ int resident_plan(const nw_grid* g, const nw_medium* m, int n_shots, int n_rec, 
       if (base > kMaxSmem) continue;
       // the shared tables hold every receiver or touched cell, should all lie in one slab
       const int cap_list = (ADJ ? n_cells : n_rec) / 4 * 4 + 4, cap_ent = ADJ ? 4 * n_rec + 4 : 0;
-      const size_t smem = base + cap_list * (ADJ ? L::cell_entry : L::list_entry) + cap_ent * L::csr_entry;
+      const size_t smem = base + cap_list * (ADJ ? L::cell_entry : L::list_entry) + cap_ent * L::csr_entry +
+                          (n_imposed ? L::lane_bytes(nv, max_rows) + n_imposed * L::imposed_entry : 0);
+      if (n_imposed > 65000) continue;  // (16-bit entries)
       if (smem > kMaxSmem - 128 || (ADJ && n_cells > 4095)) continue;  // (12 bits of a vector's table entry)
       // Cycles per step, from a sweep over grids of 117^2 to 552^2: a warp's row costs its shared-memory
       // wavefronts (no other warp's overlaps them), a thread's rows run one after the other, and a step has
@@ -620,13 +622,13 @@ int launch_resident_v(const nw::KGrid<T>& kg, const nw::Resident<T>& a, const Re
 // cluster's shared memory and registers, or has three dimensions).
 template <typename T, bool ADJ>
 int resident_for(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t, ResidentPlan* p,
-                 bool crowded = false) {
+                 bool crowded = false, int n_imposed = 0) {
   *p = ResidentPlan();
   if (g->ndim != 2) return NW_OK;
   if ((long long)a->n_rec * t->n_t > INT_MAX) return NW_OK;
   auto plan = [&](bool c) {
-    return g->radius == 1 ? resident_plan<T, 1, ADJ>(g, m, a->n_shots, a->n_rec, a->n_cells, c, p)
-                          : resident_plan<T, 2, ADJ>(g, m, a->n_shots, a->n_rec, a->n_cells, c, p);
+    return g->radius == 1 ? resident_plan<T, 1, ADJ>(g, m, a->n_shots, n_imposed ? 0 : a->n_rec, a->n_cells, n_imposed, c, p)
+                          : resident_plan<T, 2, ADJ>(g, m, a->n_shots, n_imposed ? 0 : a->n_rec, a->n_cells, n_imposed, c, p);
   };
   int rc = plan(false);
   if (rc || !p->ok) return rc;
@@ -690,8 +692,12 @@ template <typename T>
 int resident_forward(const nw_grid* g, const nw::KGrid<T>& kg, const nw_medium* m, const nw_acquisition* a,
                      const nw_time* t, const ResidentPlan& p, T* prev, T* cur, T* out_prev, T* out_cur, int n,
                      int n_end, T* traces, T* lap, T* psi, cudaStream_t s, const T* const* faces = nullptr,
-                     const nw_storage* snaps = nullptr) {
+                     const nw_storage* snaps = nullptr, const int64_t* imposed = nullptr, int n_imposed = 0,
+                     const T* imposed_tr = nullptr) {
   nw::Resident<T> r = resident_args<T>(g, m, a, t, p);
+  r.imposed = imposed;
+  r.n_imposed = n_imposed;
+  r.imposed_tr = imposed_tr;
   if (p.pml)
     for (int ax = 0; ax < 2; ++ax) {  // psi levels 2 * axis + step parity, or the given ones of step n
       r.f_in[ax] = faces ? faces[ax] : psi + (long long)(2 * ax + n % 2) * r.level;
@@ -2402,6 +2408,12 @@ int time_reversal_impl(const nw_grid* g, const nw_medium* m, const nw_acquisitio
   };
   int rc = impose(0);
   if (rc) return rc;
+  ResidentPlan res;
+  if (tu.fwd.depth != 2) rc = resident_for<T, false>(g, m, a, t, &res, false, n_cells);
+  if (rc) return rc;
+  if (res.ok && N >= kResidentSteps)  // the steps and the later levels' conditions in one launch
+    return resident_forward<T>(g, kg, m, a, t, res, L.at(-1), L.at(0), L.at(N - 1), L.at(N), 0, N, nullptr, nullptr,
+                               (T*)st->pml_psi, s, nullptr, nullptr, cells, n_cells, traces);
   for (int n = 0; n < N; ++n) {
     rc = forward_step<T>(g, kg, m, a, t, tu, L, n, nullptr, nullptr, s, (T*)st->pml_psi);
     if (rc) return rc;
