@@ -294,6 +294,14 @@ int nw_adjoint(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, co
                void* grad_acc, void* lambda0, void* mu1, void* stream);
 
 /*
+ * The adjoint run of nw_adjoint for the initial state alone (lambda0 and mu1, both required): without the
+ * velocity gradient, so it needs no history or snapshots of the forward run and reads none.
+ */
+int nw_adjoint_initial(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
+                       const nw_tuning* tune, const void* grad_traces, void* work, void* lambda0, void* mu1,
+                       void* stream);
+
+/*
  * Reduce gradient accumulators (n_acc fields in the grid's dtype holding c2dt2 * dJ/dc2dt2, as
  * nw_adjoint leaves them) in float64 and apply the chain rule of c2dt2 = pad_replicate(c)^2 dt^2: grad_c (physical
  * grid, float64) = pad_replicate^T(2 c_pad dt2 * sum_acc g / (c_pad^2 dt2))

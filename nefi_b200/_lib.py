@@ -110,6 +110,7 @@ _SIGNATURES = {
                              C.c_int32, C.c_int32, VP, VP]),
     "nw_adjoint": (C.c_int, [P(Grid), P(Medium), P(Acquisition), P(Time), P(Storage), P(Tuning), VP,
                              VP, VP, VP, VP, VP]),
+    "nw_adjoint_initial": (C.c_int, [P(Grid), P(Medium), P(Acquisition), P(Time), P(Tuning), VP, VP, VP, VP, VP]),
     "nw_reduce_grad_c": (C.c_int, [P(Grid), VP, VP, C.c_double, C.c_int32, VP, C.c_int32, VP, VP]),
     "nw_initial_state_adjoint": (C.c_int, [P(Grid), VP, P(Medium), P(Time), C.c_int32, VP, VP, VP,
                                            VP, VP, C.c_int32, VP]),

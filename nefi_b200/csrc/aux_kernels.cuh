@@ -13,6 +13,14 @@ struct PadMap {
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
+// Cell t of an n0 x n1 x n2 grid (fewer than 2^31 cells: 32-bit divisions).
+__device__ __forceinline__ void cell_of(int t, int n1, int n2, int& x, int& y, int& z) {
+  const unsigned r = (unsigned)t / (unsigned)n2;
+  z = t - (int)r * n2;
+  x = (int)(r / (unsigned)n1);
+  y = (int)r - x * n1;
+}
+
 // c2dt2[cell] = c[pad_replicate(cell)]^2 * dt2 over all padded cells (2-D: n2 = 1).
 template <typename T>
 __global__ void medium_kernel(KGrid<T> g, PadMap pm, const T* __restrict__ c, T dt2, int ndim,
@@ -20,9 +28,8 @@ __global__ void medium_kernel(KGrid<T> g, PadMap pm, const T* __restrict__ c, T 
   const long long cells = (long long)g.n0 * g.n1 * g.n2;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cells;
        t += (long long)gridDim.x * blockDim.x) {
-    const int z = (int)(t % g.n2);
-    const int y = (int)((t / g.n2) % g.n1);
-    const int x = (int)(t / ((long long)g.n2 * g.n1));
+    int x, y, z;
+    cell_of((int)t, g.n1, g.n2, x, y, z);
     long long src, dst;
     if (ndim == 2) {  // (x, y) are the two axes, z == 0
       const int i = clampi(x - pm.a0, 0, pm.m0 - 1), j = clampi(y - pm.a1, 0, pm.m1 - 1);
@@ -50,9 +57,8 @@ __global__ void pad_zero_kernel(KGrid<T> g, PadMap pm, int ndim, const T* __rest
   T* dst = lvl + (long long)s * g.field;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cells;
        t += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(t % pm.m2);
-    const int j = (int)((t / pm.m2) % pm.m1);
-    const int i = (int)(t / ((long long)pm.m2 * pm.m1));
+    int i, j, k;
+    cell_of((int)t, pm.m1, pm.m2, i, j, k);
     long long d;
     if (ndim == 2) d = g.origin + (long long)(i + pm.a0) * g.s0 + (j + pm.a1);
     else d = g.origin + (long long)(i + pm.a0) * g.s0 + (long long)(j + pm.a1) * g.s1 + (k + pm.a2);
@@ -76,14 +82,6 @@ __device__ __forceinline__ T lap_at(const KGrid<T>& g, const T* __restrict__ p, 
   return l;
 }
 
-__device__ __forceinline__ bool cell_of(long long t, int n0, int n1, int n2, int ndim, int& x, int& y,
-                                        int& z) {
-  z = (int)(t % n2);
-  y = (int)((t / n2) % n1);
-  x = (int)(t / ((long long)n2 * n1));
-  return true;
-}
-
 template <typename T>
 __device__ __forceinline__ long long ghost_index(const KGrid<T>& g, int ndim, int x, int y, int z) {
   return ndim == 2 ? g.origin + (long long)x * g.s0 + y
@@ -101,7 +99,7 @@ __global__ void initial_prev_kernel(KGrid<T> g, int ndim, const T* __restrict__ 
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cells;
        t += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
-    cell_of(t, g.n0, g.n1, g.n2, ndim, x, y, z);
+    cell_of((int)t, g.n1, g.n2, x, y, z);
     const long long i = ghost_index(g, ndim, x, y, z);
     const T h = T(0.5) * C[i];
     out[i] = p[i] + h * lap_at<T, R>(g, p, i, ndim);
@@ -130,7 +128,7 @@ __global__ void unscale_kernel(KGrid<T> g, int ndim, const T* __restrict__ C, co
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cells;
        t += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
-    cell_of(t, g.n0, g.n1, g.n2, ndim, x, y, z);
+    cell_of((int)t, g.n1, g.n2, x, y, z);
     const long long i = ghost_index(g, ndim, x, y, z);
     out[so + i] = q[so + i] / C[i];
   }
@@ -154,7 +152,7 @@ __global__ void initial_adjoint_kernel(KGrid<T> g, PadMap pm, int ndim, const T*
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cells;
        t += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
-    cell_of(t, g.n0, g.n1, g.n2, ndim, x, y, z);
+    cell_of((int)t, g.n1, g.n2, x, y, z);
     const long long i = ghost_index(g, ndim, x, y, z);
     int pi, pj, pk;
     if (ndim == 2) { pi = x - pm.a0; pj = y - pm.a1; pk = 0; }
@@ -215,9 +213,8 @@ __global__ void reduce_grad_kernel(KGrid<T> g, PadMap pm, int ndim, const T* __r
     const long long t = base + lane;
     int x0 = 0, x1 = -1, y0 = 0, y1 = 0, z0 = 0, z1 = 0;
     if (t < pcells) {
-      const int k = (int)(t % pm.m2);
-      const int j = (int)((t / pm.m2) % pm.m1);
-      const int i = (int)(t / ((long long)pm.m2 * pm.m1));
+      int i, j, k;
+      cell_of((int)t, pm.m1, pm.m2, i, j, k);
       x0 = lo(i, pm.a0, pm.m0); x1 = hi(i, pm.a0, pm.m0);
       y0 = lo(j, pm.a1, pm.m1); y1 = hi(j, pm.a1, pm.m1);
       z0 = ndim == 3 ? lo(k, pm.a2, pm.m2) : 0; z1 = ndim == 3 ? hi(k, pm.a2, pm.m2) : 0;

@@ -1185,17 +1185,18 @@ template <typename T>
 int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
                  const nw_storage* st, const Tune& tu, const T* gtr, T* work, T* gacc, T* lambda0,
                  T* mu1, cudaStream_t s, bool crowded = false) {
+  const bool velocity = gacc != nullptr;  // with the velocity gradient (else the initial state's alone)
   const int N = t->n_steps, M = t->substeps, S = a->n_shots;
   const long long LE = (long long)S * g->field_elems;
   const size_t lvl_bytes = (size_t)LE * sizeof(T);
   const nw::KGrid<T> kg = kgrid<T>(g);
   const bool ab = m->coef_a != nullptr;
   NW_CUDA(cudaMemsetAsync(work, 0, work_levels(g) * lvl_bytes, s));
-  NW_CUDA(cudaMemsetAsync(gacc, 0, (size_t)n_acc_fields(g, tu, S) * g->field_elems * sizeof(T), s));
+  if (velocity) NW_CUDA(cudaMemsetAsync(gacc, 0, (size_t)n_acc_fields(g, tu, S) * g->field_elems * sizeof(T), s));
   auto q = [&](int n) { return work + (long long)(n % 3) * LE; };  // q^n = C mu^n, three levels
-  const bool hist = st->history != nullptr;
-  const bool ckpt = !hist && st->snap != nullptr;
-  if (!hist && !ckpt && N > 0) return fail(NW_ERR_ARG, "adjoint needs a history or snapshots");
+  const bool hist = velocity && st->history != nullptr;
+  const bool ckpt = velocity && !hist && st->snap != nullptr;
+  if (velocity && !hist && !ckpt && N > 0) return fail(NW_ERR_ARG, "adjoint needs a history or snapshots");
   const int K = ckpt ? st->segment : 0;
   if (ckpt && (K < 1 || !st->ring || !st->segbuf))
     return fail(NW_ERR_ARG, "snapshots need a ring, a segment buffer and segment >= 1");
@@ -1320,9 +1321,14 @@ int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
   // A resident sweep keeps q^{n+1}, q^{n+2} in the first two work levels and one gradient sum per shot in
   // the third; lv1, lv0 are q^1 and q^0 at the end.
   T *lv0 = res.ok ? work : q(0), *lv1 = res.ok ? work + LE : q(1);
-  T* racc = res.pml ? gacc : work + 2 * LE;  // (with a PML the accumulators are per shot already)
+  T* racc = !velocity ? nullptr : res.pml ? gacc : work + 2 * LE;  // (with a PML the accumulators are per shot already)
   if (res.ok) {
-    if (hist) {
+    if (!velocity) {
+      const int rc = N >= n_stop ? resident_adjoint<T>(g, kg, m, a, t, res, work + LE, work, nullptr, N, n_stop, gtr,
+                                                       nullptr, 0, 0, work + 3 * LE, s)
+                                 : NW_OK;
+      if (rc) return rc;
+    } else if (hist) {
       const int rc = N >= n_stop ? resident_adjoint<T>(g, kg, m, a, t, res, work + LE, work, racc, N, n_stop, gtr,
                                                        (const T*)st->history, 0, N, work + 3 * LE, s)
                                  : NW_OK;
@@ -1370,9 +1376,11 @@ int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
     }
     return fail(NW_ERR_ARG, "schedule: ended before the YOUTURN of segment " + std::to_string(seg));
   };
-  for (int n = res.ok && hist ? n_stop - 1 : N - 1; n >= n_stop; --n) {
+  for (int n = res.ok && (hist || !velocity) ? n_stop - 1 : N - 1; n >= n_stop; --n) {
     const T* lap;
-    if (hist) {
+    if (!velocity) {
+      lap = nullptr;
+    } else if (hist) {
       lap = (const T*)st->history + (long long)n * LE;
     } else {
       const int n0 = (n / K) * K;
@@ -1433,7 +1441,7 @@ int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
     rc = inject3(n);
     if (rc) return rc;
   }
-  if (res.ok && !res.pml && N > 0) {  // the accumulator fields: the shots of a group summed in order
+  if (res.ok && velocity && !res.pml && N > 0) {  // the accumulator fields: the shots of a group summed in order
     const dim3 gg(grid_blocks(g->field_elems, 256), tu.adj.groups(S));
     nw::group_sum_kernel<T><<<gg, 256, 0, s>>>(work + 2 * LE, g->field_elems, S, tu.adj.spc, gacc);
     NW_LAUNCHED();
@@ -1658,6 +1666,29 @@ int nw_adjoint(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, co
                                (float*)lambda0, (float*)mu1, (cudaStream_t)stream);
   return adjoint_impl<double>(g, m, a, t, st, tu, (const double*)grad_traces, (double*)work, (double*)grad_acc,
                               (double*)lambda0, (double*)mu1, (cudaStream_t)stream);
+}
+
+int nw_adjoint_initial(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
+                       const nw_tuning* tune, const void* grad_traces, void* work, void* lambda0, void* mu1,
+                       void* stream) {
+  int rc = check_grid(g);
+  if (rc) return rc;
+  Tune tu;
+  rc = resolve_tune(g, tune, &tu);
+  if (rc) return rc;
+  const nw_storage st = {};
+  rc = check_run(g, m, a, t, &st, tu);
+  if (rc) return rc;
+  if (!grad_traces || !work || !lambda0 || !mu1) return fail(NW_ERR_ARG, "NULL adjoint buffer");
+  if (misaligned16(work) || misaligned16(lambda0) || misaligned16(mu1))
+    return fail(NW_ERR_ARG, "device buffers must start on 16-byte boundaries");
+  if (a->n_cells > 0 && (!a->cell_index || !a->cell_ptr || !a->cell_rec || !a->cell_weight))
+    return fail(NW_ERR_ARG, "receiver adjoint table is NULL");
+  if (g->dtype == NW_F32)
+    return adjoint_impl<float>(g, m, a, t, &st, tu, (const float*)grad_traces, (float*)work, nullptr, (float*)lambda0,
+                               (float*)mu1, (cudaStream_t)stream);
+  return adjoint_impl<double>(g, m, a, t, &st, tu, (const double*)grad_traces, (double*)work, nullptr, (double*)lambda0,
+                              (double*)mu1, (cudaStream_t)stream);
 }
 
 int nw_reduce_grad_c(const nw_grid* g, const int32_t* n_abs, const void* c, double dt2,
@@ -2588,7 +2619,7 @@ int run_misfit_program(const nw_traces* t, nw::MisfitArgs<T> a, cudaStream_t s, 
   const nw::fft::Groups G = nw::fft::make_groups(t->log2_len);
   const int L = 1 << t->log2_len;
   const size_t smem = (size_t)(G.tab_len + nw::fft::slot(L - 1) + 1) * sizeof(typename nw::fft::Cx<T>::t);
-  const int threads = std::min(nw::misfit_threads<T>(), std::max(32, L >> 4));
+  int threads = std::min(nw::misfit_threads<T>(), std::max(32, L >> 4));
   auto kern = nw::misfit_fft_kernel<T>;
   NW_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, sms = 0, per_sm = 0;

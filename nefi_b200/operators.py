@@ -634,8 +634,11 @@ class _PATFunction(torch.autograd.Function):
         acq = plan.acquisition(S)
         need_p0, need_c = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         needs_grad = need_p0 or need_c
+        # the gradient of p0 alone needs nothing of the forward run: it is stored for the gradient of c, or when
+        # a segment length or slot count was asked for
+        keep = need_c or (needs_grad and bool(op.checkpoint_every or op.checkpoint_slots))
         mode = (plan_storage(plan, S, op.n_steps, op.grad_mode, op.checkpoint_every, op.snapshot,
-                             op._budget(p0.device), op.checkpoint_slots) if needs_grad else ("ring", None))
+                             op._budget(p0.device), op.checkpoint_slots) if keep else ("ring", None))
         run = _Run(plan, S, op.n_steps, mode, op.snapshot)
         _lib.check(lib.nw_initial_state(C.byref(plan.g), plan.n_abs, C.byref(medium), S, p0f.data_ptr(),
                                         run.level(-1).data_ptr(), run.level(0).data_ptr(), stream))
@@ -643,9 +646,10 @@ class _PATFunction(torch.autograd.Function):
         traces = torch.empty(S, plan.n_rec, op.n_t, device=p0.device, dtype=p0.dtype)
         _forward_sweep(plan, medium, acq, run, 0, op.n_steps, traces, stream)
         if needs_grad:
-            ctx.op, ctx.run, ctx.S, ctx.batch, ctx.c2dt2, ctx.p0_level = op, run, S, batch, c2dt2, p0_level
+            ctx.op, ctx.plan, ctx.S, ctx.batch, ctx.c2dt2, ctx.p0_level = op, plan, S, batch, c2dt2, p0_level
+            ctx.run = run if keep else None
             ctx.save_for_backward(c)
-        else:
+        if not keep:
             run.release()
         return traces.reshape(*batch, plan.n_rec, op.n_t)
 
@@ -654,16 +658,22 @@ class _PATFunction(torch.autograd.Function):
     @_lib.on_device
     def backward(ctx, grad_traces: torch.Tensor):
         (c,) = ctx.saved_tensors
-        op, run, S = ctx.op, ctx.run, ctx.S
-        plan = run.plan
+        op, run, S, plan = ctx.op, ctx.run, ctx.S, ctx.plan
         dev = grad_traces.device
         stream = _lib.stream_handle(dev)
         lib = _lib.load()
         medium = plan.medium(ctx.c2dt2)
         acq = plan.acquisition(S)
         gtr = grad_traces.reshape(S, plan.n_rec, op.n_t).contiguous().to(plan.dtype)
-        gC, lam0, mu1 = _adjoint_sweep(plan, medium, acq, run, gtr, True, stream)
         need_c = ctx.needs_input_grad[1]
+        if run is not None:
+            gC, lam0, mu1 = _adjoint_sweep(plan, medium, acq, run, gtr, True, stream)
+        else:
+            work = plan.empty_levels(7 if plan.pml is not None else 3, S, zero=False)
+            lam0, mu1 = plan.empty_levels(1, S, zero=False)[0], plan.empty_levels(1, S, zero=False)[0]
+            _lib.check(lib.nw_adjoint_initial(C.byref(plan.g), C.byref(medium), C.byref(acq), C.byref(plan.time),
+                                              C.byref(plan.tuning), gtr.data_ptr(), work.data_ptr(), lam0.data_ptr(),
+                                              mu1.data_ptr(), stream))
         grad_p0 = torch.empty(S, *plan.pgrid.shape, device=dev, dtype=plan.dtype)
         p0l = ctx.p0_level if need_c else lam0
         _lib.check(lib.nw_initial_state_adjoint(C.byref(plan.g), plan.n_abs, C.byref(medium),
@@ -677,7 +687,8 @@ class _PATFunction(torch.autograd.Function):
             _lib.check(lib.nw_reduce_grad_c(C.byref(plan.g), plan.n_abs, c.contiguous().data_ptr(),
                                             op.dt**2, gC.shape[0], gC.data_ptr(), 0, g64.data_ptr(), stream))
             grad_c = g64.to(c.dtype)
-        run.release()
+        if run is not None:
+            run.release()
         ctx.run = None
         ctx.p0_level = None
         gp0 = grad_p0.reshape(*ctx.batch, *plan.pgrid.shape) if ctx.needs_input_grad[0] else None
