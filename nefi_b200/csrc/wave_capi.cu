@@ -412,21 +412,29 @@ int launch_adj2_v(const nw::KGrid<T>& kg, const nw::Tiled2<T>& st, dim3 grid, cu
   return launch_pdl(nw::adj2d<T, R, VZ, RX, AB>, grid, smem, s, kg, whole_grid(kg, st));
 }
 
-// 3-D step: forward (ADJ = false) or adjoint, plane-marching tiles of 8 x 64 (y, z) cells over chunks
-// of kXChunk planes (16-row tiles of 16 warps measured 7 % slower on the 256^3 photoacoustic gradient).
-constexpr int kXChunk = 32;
+// 3-D step: forward (ADJ = false) or adjoint. The tile splits a row into equal parts of at most 40 vectors and
+// takes the rows that 256 threads then cover; the chunk of planes per CTA is the one whose waves (three CTAs
+// per SM) march the fewest planes, the chunk's halo planes included.
 template <typename T, int R, bool ADJ>
 int launch_step3_r(const nw_grid* g, const nw::KGrid<T>& kg, const nw::Step3<T>& st, int n_shots, cudaStream_t s) {
-  using S = nw::Tile3Shape<T, 2, R>;
-  const int tz = (g->n[2] + S::TZ - 1) / S::TZ, ty = (g->n[1] + S::TY - 1) / S::TY;
-  if ((long long)tz * ty * n_shots > INT_MAX) return fail(NW_ERR_UNSUPPORTED, "3-D grid: too many tiles x shots");
-  const dim3 grid((unsigned)((long long)tz * ty * n_shots), (g->n[0] + kXChunk - 1) / kXChunk);  // shot fastest
-  constexpr size_t smem = (size_t)S::NSP * S::PS * sizeof(T);
-  static_assert(smem <= kMaxSmem, "plane ring above the shared-memory limit");
-  static bool done = false;
-  int rc = allow_smem(nw::step3t<T, R, 2, ADJ>, smem, &done);
-  if (rc) return rc;
-  return launch_pdl_b(nw::step3t<T, R, 2, ADJ>, grid, dim3(S::NT), smem, s, kg, st, kXChunk, n_shots);
+  using S = nw::Tile3Shape<T, R>;
+  const int n_vec = (g->n[2] + S::VZ - 1) / S::VZ, parts = (n_vec + 39) / 40, wv = (n_vec + parts - 1) / parts;
+  const int ty = std::min(S::NT / wv, S::NCH * S::NT / (wv + 2) - 2 * R);
+  const long long tiles = (long long)((n_vec + wv - 1) / wv) * ((g->n[1] + ty - 1) / ty) * n_shots;
+  if (tiles > INT_MAX) return fail(NW_ERR_UNSUPPORTED, "3-D grid: too many tiles x shots");
+  int xc = 0;
+  long long best = LLONG_MAX;
+  for (int c = 8; c <= 64; ++c) {
+    const long long ctas = tiles * ((g->n[0] + c - 1) / c), waves = (ctas + 3 * 148 - 1) / (3 * 148);
+    const long long planes = waves * (std::min(c, (int)g->n[0]) + 2 * R + 1);
+    if (planes < best) {
+      best = planes;
+      xc = c;
+    }
+  }
+  const dim3 grid((unsigned)tiles, (g->n[0] + xc - 1) / xc);  // shot fastest
+  const size_t smem = (size_t)S::NSP * S::plane(wv, ty) * sizeof(T);  // (at most 40 KB)
+  return launch_pdl_b(nw::step3t<T, R, ADJ>, grid, dim3(S::NT), smem, s, kg, st, wv, ty, xc, n_shots);
 }
 template <typename T, bool ADJ>
 int launch_step3(const nw_grid* g, const nw::KGrid<T>& kg, const nw::Step3<T>& st, bool ab, int n_shots,
