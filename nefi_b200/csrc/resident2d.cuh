@@ -15,11 +15,17 @@
 // row of p^n after that read, so nobody reads the rows any more. Waits are bounded: one that gives up sets the
 // device status word and puts a NaN into the field, and the kernel runs on without waiting.
 //
-// Threads: a row has NV vectors of VZ = 16 / sizeof(T) columns, a slab S strips of rows; thread t steps
-// vector t % NV of strip t / NV, marching over at most RX rows with a (2R+1)-row register window. The
-// last strip marches upwards, so that both of a slab's edges are computed, and sent, first. One or more
-// further warps serve the others: they sample the receivers, gather the next step's cotangents, arm the
-// mbarriers. A warp without layer cells steps its rows without the layer's coefficients.
+// Threads: a row has NV vectors of VZ = 16 / sizeof(T) columns, a slab S strips of rows; a thread steps one
+// vector of one strip, marching over at most RX rows with a (2R+1)-row register window. The vectors that hold
+// layer columns are the last warps' (strip by strip), the others come before them, so that few warps of a slab
+// between the layers step layer cells: interleaved, 5 of the 13 warps of a 552-column slab did, and the
+// others waited for them (PML 296^2, 16 shots, adjoint: 12.4 -> 10.2 us a step). The last strip marches
+// upwards, so that both of a slab's edges are computed, and sent, first. One or more further warps serve the
+// others: they sample the receivers, gather the next step's cotangents, arm the mbarriers. A warp without
+// layer cells steps its rows without the layer's coefficients.
+//
+// Per-step time (fp32, order 4, one-step launches -> resident): 168^2 1 shot 3.45 -> 1.34 us forward, 2.48 -> 1.47
+// adjoint; 296^2 4 shots 3.58 -> 1.99, 4.96 -> 2.29; 440^2 10 shots 6.81 -> 5.1; 552^2 16 shots 16.4 -> 13.5.
 //
 // The arithmetic of a cell is that of fwd2d / adj2d, operation by operation: fields and traces are
 // bitwise those of the one-step launches. The gradient is summed per shot over the steps.
@@ -100,7 +106,14 @@ struct Resident {
 // Threads per CTA at most: 16 warps leave each 128 registers, which hold c^2 dt^2 and, in the adjoint, the
 // gradient sums of RX vectors beside the 2R+1-row window (more warps would spill them).
 // A PML's strips hold more beside them: 12 warps of 168 registers.
-constexpr int resident_threads(bool pml) { return pml ? 384 : 512; }
+__host__ __device__ constexpr int resident_threads(bool pml) { return pml ? 384 : 512; }
+
+// Threads that step cells: the vectors without layer columns of all strips, then the others, each rounded up to
+// warps.
+__host__ __device__ inline int resident_cell_threads(int nv, int edge_lo, int edge_hi, int strips) {
+  const int n_in = edge_hi - edge_lo;
+  return (strips * n_in + 31) / 32 * 32 + (strips * (nv - n_in) + 31) / 32 * 32;
+}
 
 // Shared memory: two levels of the slab with R halo rows above and below (a zero vector before the first
 // row and after each row), the mbarriers, then the tables.
@@ -209,7 +222,8 @@ __device__ __forceinline__ int2 count_below(const int64_t* idx, int n, long long
   return total;
 }
 
-template <typename T, int R, int RX, bool ADJ, bool PML>
+// IMP: the forward of a time reversal, which imposes cells after each step (apart: it costs registers).
+template <typename T, int R, int RX, bool ADJ, bool PML, bool IMP>
 __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __grid_constant__ KGrid<T> g, const __grid_constant__ Resident<T> a) {
   using L = ResidentSmem<T, R>;
   constexpr int VZ = L::VZ;
@@ -232,9 +246,13 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
   const bool has_up = rank > 0, has_dn = rank + 1 < a.cluster;
 
   // ---- this thread's strip
-  const int strip = tid / a.nv, vec = tid - strip * a.nv;
-  const bool work = strip < a.strips;
-  const int svc = (a.strips * a.nv + 31) / 32 * 32;  // first service thread: the warps that step no cells
+  const int svc = resident_cell_threads(a.nv, a.edge_lo, a.edge_hi, a.strips);  // first service thread
+  const int n_in = a.edge_hi - a.edge_lo, in_thr = (a.strips * n_in + 31) / 32 * 32, n_edge_vec = a.nv - n_in;
+  const bool edge_thr = tid >= in_thr;
+  const int strip = edge_thr ? (tid - in_thr) / max(n_edge_vec, 1) : tid / max(n_in, 1);
+  const int in_group = edge_thr ? tid - in_thr - strip * n_edge_vec : tid - strip * n_in;
+  const int vec = !edge_thr ? a.edge_lo + in_group : in_group < a.edge_lo ? in_group : in_group - a.edge_lo + a.edge_hi;
+  const bool work = tid < svc && strip < a.strips;
   const int ra = work ? rows * strip / a.strips : 0;
   const int rb = work ? rows * (strip + 1) / a.strips : 0;
   const int nr = rb - ra;                                 // rows of the strip (<= RX)
@@ -428,7 +446,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
     }
   };
   if constexpr (!ADJ) {
-    if (a.imposed) {
+    if constexpr (IMP) {
       for (int i = tid; i < a.nv * rows * VZ; i += nthr) lane_map[i] = 0;
       __syncthreads();
       for (int c = tid; c < a.n_imposed; c += nthr) {
@@ -551,17 +569,21 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
     for (int k = 0; k < PF && k < RX; ++k)
       if (lap_now && k < nr) vldcg<T, VZ>(lap_now + k * dld, lpb[k]);
   }
-  // R edge rows of this thread's vector's piece (the lanes of this warp in the same strip: one piece of a row,
-  // sent by its first lane) of the new level into the halo rows of the CTA above (side 0) or below. A shared
+  // R edge rows of this thread's vector's piece (the lanes of this warp with adjoining vectors of the same strip:
+  // one piece of a row, sent by its first lane) of the new level into the halo rows of the CTA above (side 0) or below. A shared
   // address of this CTA and the same one of a neighbour differ by a constant; row r of this slab is row r + R of
   // theirs below the slab above's last one, and row r - (rows - R) of the slab below.
   const unsigned up_off = has_up ? map_cta(mbar_a, rank - 1) - mbar_a : 0, dn_off = has_dn ? map_cta(mbar_a, rank + 1) - mbar_a : 0;
-  const int seg_first = max(0, (tid & 31) - vec), seg_end = min(32, (tid & 31) - vec + a.nv);
+  const int run_lo = !edge_thr ? a.edge_lo : vec < a.edge_lo ? 0 : a.edge_hi, run_hi = !edge_thr ? a.edge_hi : vec < a.edge_lo ? a.edge_lo : a.nv;
+  __shared__ unsigned short seg_sh[resident_threads(PML)];  // first and end lane of a thread's piece
+  seg_sh[tid] = (unsigned short)(max(0, (tid & 31) - (vec - run_lo)) | min(32, (tid & 31) + run_hi - vec) << 8);
+  __syncthreads();
   auto send_rows = [&](int side, bool upwards, int m, int level) {
+    const int seg = seg_sh[threadIdx.x], seg_first = seg & 255, seg_end = seg >> 8;
     const unsigned mask = (seg_end == 32 ? ~0u : (1u << seg_end) - 1) & ~((1u << seg_first) - 1);
     fence_async();
     __syncwarp(mask);
-    if ((tid & 31) != seg_first) return;
+    if (((int)threadIdx.x & 31) != seg_first) return;
     const int row_b = pitch * (int)sizeof(T);
     const unsigned own = smem_addr(buf) + zc * (unsigned)sizeof(T) + level * (unsigned)(BS * (int)sizeof(T));
     const unsigned to = own + (side ? dn_off + (R - rows) * row_b : up_off + (R + X0 - a.slab[rank - 1]) * row_b);
@@ -577,6 +599,30 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
   const bool sampled = !ADJ && a.traces != nullptr;
   cluster_barrier();  // every level read, every mbarrier initialised
 
+  // The shot's source onto a vector of slab row r.
+  auto add_source = [&](int r, int m, T (&o)[VZ]) {
+    const int dx = r + X0 - a.src_corner[2 * s], z0 = zc - a.src_corner[2 * s + 1];
+    const T* w = src_sh + 4 * (m & 1) + 2 * dx;
+#pragma unroll
+    for (int v = 0; v < VZ; ++v)
+      if ((unsigned)(z0 + v) <= 1u) o[v] = add_rn(o[v], w[z0 + v]);
+  };
+  // Whether the edge rows may be sent as soon as they are marched over: not where cells are still to change
+  // after the march, the source of a warp without the layer or a time reversal's cells, in this or another
+  // thread of the piece.
+  const bool early = ADJ || (!IMP && __all_sync(0xffffffffu, rare == 0));
+  // Time reversal: the imposed cells of this strip's new level, before its edge rows are sent.
+  auto impose = [&](int m, int level) {
+    for (unsigned left = rare; left; left &= left - 1) {
+      const int r = r0 + dir * (__ffs(left) - 1);
+      T* row = buf + level * BS + (R + r) * pitch + zc;
+#pragma unroll
+      for (int v = 0; v < VZ; ++v) {
+        const int e = lane_map[r * a.nv * VZ + zc + v];
+        if (e) row[v] = i_val[(m & 1) * a.n_imposed + e - 1];
+      }
+    }
+  };
   // This strip's rows of p^{n-1}, p^n and the face fields before step m, to the snapshot of step n.
   auto snapshot = [&](int m, int n) {
     T* dst = a.snap + (long long)(n / a.segment) * a.snap_stride + so + cell0;
@@ -632,7 +678,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
       T wv[2 * R + 1][VZ];
 #pragma unroll
       for (int q = 0; q < 2 * R; ++q) vload<T, VZ>(pc + (q - R) * dpo, wv[q]);
-      const unsigned now = (!ADJ || (inject && phase_c == 0)) ? rare : 0u;
+      const unsigned now = (ADJ ? inject && phase_c == 0 : a.src_corner != nullptr) ? rare : 0u;
       [[maybe_unused]] T* lps = lpo;
       [[maybe_unused]] int off = PF * dl;  // from the march's first row to the next one whose Lap p is loaded
       const bool first = n == 0 && (ADJ || a.first_b_one);
@@ -693,25 +739,10 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
           }
         }
         v_fma(cc[C_REG ? k : k % PF], lp, two, o);
-        if constexpr (!ADJ) {
-          if (a.src_corner && (now >> k & 1u)) {  // the source
-            const int dx = r0 + dir * k + X0 - a.src_corner[2 * s], z0 = zc - a.src_corner[2 * s + 1];
-            const T* w = src_sh + 4 * (m & 1) + 2 * dx;
-#pragma unroll
-            for (int v = 0; v < VZ; ++v)
-              if ((unsigned)(z0 + v) <= 1u) o[v] = add_rn(o[v], w[z0 + v]);
-          }
+        if constexpr (!ADJ && LAYER) {
+          if (now >> k & 1u) add_source(r0 + dir * k, m, o);
         }
         if constexpr (LAYER) v_mul(ca, o, o);
-        if constexpr (!ADJ) {
-          if (a.imposed && (now >> k & 1u)) {
-#pragma unroll
-            for (int v = 0; v < VZ; ++v) {
-              const int e = lane_map[(r0 + dir * k) * a.nv * VZ + zc + v];
-              if (e) o[v] = i_val[(m & 1) * a.n_imposed + e - 1];
-            }
-          }
-        }
         vstore<T, VZ>(out, o);
         if constexpr (!ADJ) {
           if (lps) {  // (whole vectors: nothing reads the ghost columns of a stored Laplacian)
@@ -726,7 +757,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
           if (!C_REG && k + PF < RX && k + PF < nr) vldg<T, VZ>(a.C + first_cell + off, cc[k % PF]);
           off += dl;
         }
-        if (k == R - 1 && !last) {  // the slab's edge rows are done: on their way while the rest is stepped
+        if (k == R - 1 && !last && early) {  // the slab's edge rows are done: on their way while the rest is stepped
           if (send_up) send_rows(0, false, m, level);
           if (send_dn) send_rows(1, true, m, level);
         }
@@ -734,6 +765,21 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
         for (int q = 0; q < 2 * R; ++q)
 #pragma unroll
           for (int v = 0; v < VZ; ++v) wv[q][v] = wv[q + 1][v];
+      }
+      if (!early) {
+        if constexpr (IMP) impose(m, level);
+        else if (!ADJ && !LAYER && now) {  // the source, onto the stored cells (A = 1)
+          for (unsigned left = now; left; left &= left - 1) {
+            const int r = r0 + dir * (__ffs(left) - 1);
+            T* row = buf + level * BS + (R + r) * pitch + zc;
+            T o[VZ];
+            vload<T, VZ>(row, o);
+            add_source(r, m, o);
+            vstore<T, VZ>(row, o);
+          }
+        }
+        if (send_up && !last) send_rows(0, false, m, level);
+        if (send_dn && !last) send_rows(1, true, m, level);
       }
       if (send_late && !last) send_rows(1, false, m, level);
       if constexpr (ADJ) {
@@ -783,7 +829,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
         T* f0 = psi0 + r0 * pitch + zc;
         const T* f1o = psi1 + ((m & 1) * a.max_rows + r0) * pitch + zc;
         T* f1n = psi1 + ((1 - (m & 1)) * a.max_rows + r0) * pitch + zc;
-        const unsigned now = (!ADJ || (inject && phase_c == 0)) ? rare : 0u;
+        const unsigned now = (ADJ ? inject && phase_c == 0 : a.src_corner != nullptr) ? rare : 0u;
         [[maybe_unused]] T* lps = lpo;
         [[maybe_unused]] int off = PF * dl;
         int cell = first_cell;
@@ -929,22 +975,9 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
               lp[v] = add_rn(lp[v], px[v]);
               o[v] = fma_rn(-cZ[v], wv[R][v], fma_rn(cc[k][v], lp[v], fma_rn(-cB[v], pv[v], add_rn(wv[R][v], wv[R][v]))));
             }
-            if (a.src_corner && (now >> k & 1u)) {  // the source
-              const int dx = r0 + k + X0 - a.src_corner[2 * s], z0 = zc - a.src_corner[2 * s + 1];
-              const T* wgt = src_sh + 4 * (m & 1) + 2 * dx;
-#pragma unroll
-              for (int v = 0; v < VZ; ++v)
-                if ((unsigned)(z0 + v) <= 1u) o[v] = add_rn(o[v], wgt[z0 + v]);
-            }
+            if (now >> k & 1u) add_source(r0 + k, m, o);
 #pragma unroll
             for (int v = 0; v < VZ; ++v) o[v] = mul_rn(cA[v], o[v]);
-            if (a.imposed && (now >> k & 1u)) {
-#pragma unroll
-              for (int v = 0; v < VZ; ++v) {
-                const int e = lane_map[(r0 + k) * a.nv * VZ + zc + v];
-                if (e) o[v] = i_val[(m & 1) * a.n_imposed + e - 1];
-              }
-            }
             if (lps) {
               vstore<T, VZ>(lps, lp);
               lps += dl;
@@ -971,7 +1004,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
             off += dl;
           }
           vstore<T, VZ>(pn, o);
-          if (k == R - 1 && !last && send_up) send_rows(0, false, m, level);
+          if (k == R - 1 && !last && early && send_up) send_rows(0, false, m, level);
           pc += dpo;
           pn += dpo;
           f1o += dpo;
@@ -982,6 +1015,10 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
           for (int q = 0; q < 2 * R; ++q)
 #pragma unroll
             for (int v = 0; v < VZ; ++v) wv[q][v] = wv[q + 1][v];
+        }
+        if (!early) {
+          if constexpr (IMP) impose(m, level);
+          if (send_up && !last) send_rows(0, false, m, level);
         }
         if (send_late && !last) send_rows(1, false, m, level);
         if constexpr (ADJ) {
@@ -1052,7 +1089,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
           src_sh[4 * (1 - (m & 1)) + id] = mul_rn(weight, wave);
           if (m + 2 < a.count) wave = a.wavelet[n + 2];
         }
-        if (a.imposed && !last) imposed_values(n + 2, i_val + (1 - (m & 1)) * a.n_imposed, id, ns);
+        if constexpr (IMP) if (!last) imposed_values(n + 2, i_val + (1 - (m & 1)) * a.n_imposed, id, ns);
         if (++phase == a.substeps) { phase = 0; ++j; }
       }
       cta_barrier();

@@ -481,10 +481,10 @@ int cluster_slots(int size, int* out) {
   if (dev < 0 || dev >= 64) return fail(NW_ERR_UNSUPPORTED, "device index above 63");
   std::lock_guard<std::mutex> lock(mu);
   if (slots[dev][size] == 0) {
-    auto k = nw::resident2d<float, 1, 2, false, false>;
+    auto k = nw::resident2d<float, 1, 2, false, false, false>;
     const int smem = 200 * 1024;
     NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem - 128));
+    NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem - 1280));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(size);
     cfg.blockDim = dim3(256);
@@ -504,7 +504,7 @@ int cluster_slots(int size, int* out) {
 }
 
 constexpr int kResidentSteps = 3;  // fewest forward steps worth loading the state for
-constexpr int kPmlRows = 6;  // at most, with a PML (registers)
+constexpr int kPmlRows = 6;  // at most, with a PML or a time reversal (registers)
 constexpr int kResidentRows[] = {2, 4, 6, 8, 12};  // rows per thread the resident kernels are built for
 
 // How a resident sweep covers the device (see resident2d.cuh).
@@ -529,7 +529,7 @@ int resident_plan(const nw_grid* g, const nw_medium* m, int n_shots, int n_rec, 
   const int z0 = pml ? m->pml_core[2] : g->core_lo[1], z1 = pml ? m->pml_core[3] : g->core_hi[1];
   if (x0 < 0 || z0 < 0 || x1 < x0 || z1 < z0 || x1 > n0 || z1 > g->n[1]) return fail(NW_ERR_ARG, "medium.pml_core lies outside the grid");
   int edge_lo = (z0 + L::VZ - 1) / L::VZ, edge_hi = z1 / L::VZ;
-  if (edge_lo >= edge_hi) edge_lo = edge_hi = nv;
+  if (edge_lo >= edge_hi || g->absorbing == NW_ABS_NONE) edge_lo = 0, edge_hi = g->absorbing == NW_ABS_NONE ? nv : 0;
   const int ne = edge_lo + nv - edge_hi;
   auto coef_per_row = [&](int rows) {
     return pml ? L::pml_bytes(ne, nv, rows) : g->absorbing == NW_ABS_NONE ? (size_t)0 : L::coef_bytes(ne, rows);
@@ -542,11 +542,11 @@ int resident_plan(const nw_grid* g, const nw_medium* m, int n_shots, int n_rec, 
     if (rc) return rc;
     if (slots < 1) continue;
     for (int rx : kResidentRows) {
-      if (pml && rx > kPmlRows) continue;
+      if ((pml || n_imposed) && rx > kPmlRows) continue;
       for (int strips = (max_rows + rx - 1) / rx; strips <= min_rows / R && (strips - 1) * rx < 2 * max_rows; ++strips) {  // of R rows or more
       // one service warp for every 64 receivers (touched cells) of an evenly loaded slab, up to four
       const int serve = std::max(1, std::min(4, (ADJ ? n_cells : n_rec) / (64 * nc)));
-      const int cells = (strips * nv + 31) / 32 * 32;
+      const int cells = nw::resident_cell_threads(nv, edge_lo, edge_hi, strips);
       const int threads = std::min(cells + 32 * serve, nw::resident_threads(pml));
       if (threads < cells + 32) continue;
       const size_t base = L::tables(nv, max_rows, levels) + (ADJ ? L::map_bytes(nv, max_rows) : 0) + coef_per_row(max_rows);
@@ -556,13 +556,13 @@ int resident_plan(const nw_grid* g, const nw_medium* m, int n_shots, int n_rec, 
       const size_t smem = base + cap_list * (ADJ ? L::cell_entry : L::list_entry) + cap_ent * L::csr_entry +
                           (n_imposed ? L::lane_bytes(nv, max_rows) + n_imposed * L::imposed_entry : 0);
       if (n_imposed > 65000) continue;  // (16-bit entries)
-      if (smem > kMaxSmem - 128 || (ADJ && n_cells > 4095)) continue;  // (12 bits of a vector's table entry)
+      if (smem > kMaxSmem - 1280 || (ADJ && n_cells > 4095)) continue;  // (12 bits of a vector's table entry)
       // Cycles per step, from a sweep over grids of 117^2 to 552^2: a warp's row costs its shared-memory
       // wavefronts (no other warp's overlaps them), a thread's rows run one after the other, and a step has
       // its barriers and the halo's way to the neighbour. The adjoint's tallest strips, and a PML's, spill.
       const int nr = (max_rows + strips - 1) / strips;
       const double row = pml ? (ADJ ? (rx <= 4 ? 150.0 : 240.0) : 90.0) : ADJ ? (rx <= 8 ? 72.0 : 84.0) : 52.0;
-      const double chain = nr * (pml ? 750.0 : 250.0);
+      const double chain = nr * (pml ? 750.0 : 600.0);
       const double step = std::max(cells / 32 * nr * row, chain) + (nc > 1 ? 900.0 : 400.0);
       // beside other sweeps that fill the device, what counts is the SMs' time
       const double rounds = crowded ? (double)n_shots / slots : std::ceil((double)n_shots / slots);
@@ -579,16 +579,16 @@ int resident_plan(const nw_grid* g, const nw_medium* m, int n_shots, int n_rec, 
   return NW_OK;
 }
 
-template <typename T, int R, int RX, bool ADJ, bool PML>
+template <typename T, int R, int RX, bool ADJ, bool PML, bool IMP = false>
 int launch_resident_r(const nw::KGrid<T>& kg, const nw::Resident<T>& a, const ResidentPlan& p, int n_shots,
                       cudaStream_t s) {
-  auto k = nw::resident2d<T, R, RX, ADJ, PML>;
+  auto k = nw::resident2d<T, R, RX, ADJ, PML, IMP>;
   static std::atomic<bool> done[64];
   int dev = 0;
   NW_CUDA(cudaGetDevice(&dev));
   if (!done[dev & 63].load()) {
     NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem - 128));
+    NW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem - 1280));
     done[dev & 63].store(true);
   }
   cudaLaunchConfig_t cfg = {};
@@ -610,6 +610,22 @@ int launch_resident_r(const nw::KGrid<T>& kg, const nw::Resident<T>& a, const Re
 template <typename T, int R, bool ADJ>
 int launch_resident_v(const nw::KGrid<T>& kg, const nw::Resident<T>& a, const ResidentPlan& p, int n_shots,
                       cudaStream_t s) {
+  if constexpr (!ADJ) {
+    if (a.imposed) {
+      if (p.pml) {
+        switch (p.rx) {
+          case 2: return launch_resident_r<T, R, 2, ADJ, true, true>(kg, a, p, n_shots, s);
+          case 4: return launch_resident_r<T, R, 4, ADJ, true, true>(kg, a, p, n_shots, s);
+          default: return launch_resident_r<T, R, 6, ADJ, true, true>(kg, a, p, n_shots, s);
+        }
+      }
+      switch (p.rx) {
+        case 2: return launch_resident_r<T, R, 2, ADJ, false, true>(kg, a, p, n_shots, s);
+        case 4: return launch_resident_r<T, R, 4, ADJ, false, true>(kg, a, p, n_shots, s);
+        default: return launch_resident_r<T, R, 6, ADJ, false, true>(kg, a, p, n_shots, s);
+      }
+    }
+  }
   if (p.pml) {
     switch (p.rx) {
       case 2: return launch_resident_r<T, R, 2, ADJ, true>(kg, a, p, n_shots, s);
