@@ -14,9 +14,18 @@
 // group of an inverse FFT and of the next forward FFT touch the same indices, so the pointwise work
 // between two filters (subtract the observation, square and mask, crop to n) happens in registers
 // inside that merged pass. Global memory is touched once per trace for each input and output.
+//
+// What bounds it: the issue of the butterflies and the shared-memory passes between barriers, not memory. So a
+// length of 4m + 1 bits takes its lowest radix-2 stage with the radix-16 group above it, 32 elements to a thread
+// (two passes and two barriers less per filter); the samples beyond L / 2, which are zero (L >= 2n), are neither
+// formed nor transformed back; and a CTA has 256 threads where two fit an SM, so that each holds its elements in
+// registers. 16 shots of 512 traces of 4001 samples, float32, normaliser, misfit and adjoint source (five filters):
+// 1930 -> 1390 us.
 #pragma once
 
 #include <cstdint>
+
+#include "kernels.cuh"
 
 namespace nw {
 namespace fft {
@@ -25,24 +34,31 @@ template <typename T> struct Cx;
 template <> struct Cx<float> { using t = float2; };
 template <> struct Cx<double> { using t = double2; };
 
-template <typename T>
+// NAMED: with the operations named, for the passes whose products the compiler would fuse in another order from one
+// build to the next (the misfit is returned in float64, so a change of rounding shows).
+template <typename T, bool NAMED>
 __device__ __forceinline__ typename Cx<T>::t cmul(typename Cx<T>::t a, typename Cx<T>::t b) {
+  if constexpr (NAMED) return {fma_rn(a.x, b.x, -mul_rn(a.y, b.y)), fma_rn(a.y, b.x, mul_rn(a.x, b.y))};
   return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x};
 }
-template <typename T>
+template <typename T, bool NAMED>
 __device__ __forceinline__ typename Cx<T>::t cmulc(typename Cx<T>::t a, typename Cx<T>::t b) {  // a * conj(b)
+  if constexpr (NAMED) return {fma_rn(a.x, b.x, mul_rn(a.y, b.y)), fma_rn(a.y, b.x, -mul_rn(a.x, b.y))};
   return {a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y};
 }
 
 __device__ __forceinline__ void sincos_pi(float x, float* s, float* c) { sincospif(x, s, c); }
 __device__ __forceinline__ void sincos_pi(double x, double* s, double* c) { sincospi(x, s, c); }
 
-// shared-memory slot of element i: one pad slot every 16 elements spreads strided groups over banks
-__host__ __device__ __forceinline__ int slot(int i) { return i + (i >> 4); }
+// shared-memory slot of element i: one pad slot every 2^pad elements (those a thread of the lowest pass holds)
+// spreads strided groups over banks
+__host__ __device__ __forceinline__ int slot(int i, int pad) { return i + (i >> pad); }
 
 // Stage groups, top (most significant bits) first: group j covers bits [sbit, sbit + nb).
 struct Groups {
   int log2_len, count;
+  int merged;  // 1: the lowest pass takes the lowest two groups (of 4 bits and of 1) together
+  int pad;     // see slot()
   int sbit[8], nb[8], tab_off[16];  // tab_off[t]: offset of stage t's twiddles W_{2^{t+1}}^l, l < 2^sbit
   int tab_len;
 };
@@ -58,6 +74,8 @@ __host__ __device__ inline Groups make_groups(int log2_len) {
     ++g.count;
     hi -= nb;
   }
+  g.merged = g.count >= 3 && g.nb[g.count - 1] == 1;
+  g.pad = g.merged ? 5 : 4;
   int off = 16;  // the first 16 entries hold W_16^j, j < 8 (the in-group factors), padded
   for (int t = 0; t < log2_len; ++t) {
     int sb = 0;
@@ -88,8 +106,9 @@ __device__ void build_tables(const Groups& G, typename Cx<T>::t* tab) {
   }
 }
 
-// Forward (DIF) stages of one group held in v[0..2^NB): stage t = sbit + u for u = NB-1 .. 0.
-template <typename T, int NB>
+// Forward (DIF) stages of one group held in v[0..2^NB): stage t = sbit + u for u = NB-1 .. 0. HALF: the upper half of
+// v is zero and not read.
+template <typename T, int NB, bool HALF = false, bool NAMED = false>
 __device__ __forceinline__ void dif_group(typename Cx<T>::t* v, int low, int sbit, const Groups& G,
                                           const typename Cx<T>::t* tab) {
   using C = typename Cx<T>::t;
@@ -100,19 +119,23 @@ __device__ __forceinline__ void dif_group(typename Cx<T>::t* v, int low, int sbi
 #pragma unroll
     for (int k = 0; k < (1 << NB); ++k) {
       if (k & half) continue;
-      const C a = v[k], b = v[k + half];
-      v[k] = {a.x + b.x, a.y + b.y};
-      const C d = {a.x - b.x, a.y - b.y};
+      C d = v[k];
+      if (!HALF || u < NB - 1) {
+        const C a = v[k], b = v[k + half];
+        v[k] = {a.x + b.x, a.y + b.y};
+        d = {a.x - b.x, a.y - b.y};
+      }
       const int j = k & (half - 1);
       C w = wl;
-      if (j) w = cmul<T>(wl, tab[j << (3 - u)]);
-      v[k + half] = cmul<T>(d, w);
+      if (j) w = cmul<T, NAMED>(wl, tab[j << (3 - u)]);
+      v[k + half] = cmul<T, NAMED>(d, w);
     }
   }
 }
 
-// Inverse (DIT, conjugate twiddles) stages of one group: stage t = sbit + u for u = 0 .. NB-1.
-template <typename T, int NB>
+// Inverse (DIT, conjugate twiddles) stages of one group: stage t = sbit + u for u = 0 .. NB-1. HALF: the upper half
+// of the result is not wanted.
+template <typename T, int NB, bool HALF = false, bool NAMED = false>
 __device__ __forceinline__ void dit_group(typename Cx<T>::t* v, int low, int sbit, const Groups& G,
                                           const typename Cx<T>::t* tab) {
   using C = typename Cx<T>::t;
@@ -125,11 +148,11 @@ __device__ __forceinline__ void dit_group(typename Cx<T>::t* v, int low, int sbi
       if (k & half) continue;
       const int j = k & (half - 1);
       C w = wl;
-      if (j) w = cmul<T>(wl, tab[j << (3 - u)]);
+      if (j) w = cmul<T, NAMED>(wl, tab[j << (3 - u)]);
       const C a = v[k];
-      const C b = cmulc<T>(v[k + half], w);
+      const C b = cmulc<T, NAMED>(v[k + half], w);
       v[k] = {a.x + b.x, a.y + b.y};
-      v[k + half] = {a.x - b.x, a.y - b.y};
+      if (!HALF || u < NB - 1) v[k + half] = {a.x - b.x, a.y - b.y};
     }
   }
 }
@@ -209,15 +232,30 @@ __device__ __forceinline__ void apply_op(const MisfitArgs<T>& a, const PairCtx<T
   }
 }
 
+// Elements base + (k << sbit) of a group: their slots are evenly spaced where the pad repeats within a stride.
 template <typename T, int NB>
-__device__ __forceinline__ void load_group(const typename Cx<T>::t* s, typename Cx<T>::t* v, int base, int sbit) {
+__device__ __forceinline__ void load_group(const typename Cx<T>::t* s, typename Cx<T>::t* v, int base, int sbit, int pad) {
+  if (sbit >= pad) {
+    const typename Cx<T>::t* p = s + fft::slot(base, pad);
+    const int step = fft::slot(1 << sbit, pad);
 #pragma unroll
-  for (int k = 0; k < (1 << NB); ++k) v[k] = s[fft::slot(base + (k << sbit))];
+    for (int k = 0; k < (1 << NB); ++k) v[k] = p[k * step];
+  } else {
+#pragma unroll
+    for (int k = 0; k < (1 << NB); ++k) v[k] = s[fft::slot(base + (k << sbit), pad)];
+  }
 }
 template <typename T, int NB>
-__device__ __forceinline__ void store_group(typename Cx<T>::t* s, const typename Cx<T>::t* v, int base, int sbit) {
+__device__ __forceinline__ void store_group(typename Cx<T>::t* s, const typename Cx<T>::t* v, int base, int sbit, int pad) {
+  if (sbit >= pad) {
+    typename Cx<T>::t* p = s + fft::slot(base, pad);
+    const int step = fft::slot(1 << sbit, pad);
 #pragma unroll
-  for (int k = 0; k < (1 << NB); ++k) s[fft::slot(base + (k << sbit))] = v[k];
+    for (int k = 0; k < (1 << NB); ++k) p[k * step] = v[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < (1 << NB); ++k) s[fft::slot(base + (k << sbit), pad)] = v[k];
+  }
 }
 
 // One pass of group j (not the top one, not the last one) over all groups: DIF or DIT.
@@ -230,10 +268,10 @@ __device__ __forceinline__ void inner_pass(typename Cx<T>::t* s, const fft::Grou
     const int low = gi & ((1 << sbit) - 1);
     const int base = ((gi >> sbit) << (sbit + 4)) | low;
     typename Cx<T>::t v[16];
-    load_group<T, 4>(s, v, base, sbit);
-    if (DIF) fft::dif_group<T, 4>(v, low, sbit, G, tab);
-    else fft::dit_group<T, 4>(v, low, sbit, G, tab);
-    store_group<T, 4>(s, v, base, sbit);
+    load_group<T, 4>(s, v, base, sbit, G.pad);
+    if (DIF) fft::dif_group<T, 4, false, true>(v, low, sbit, G, tab);
+    else fft::dit_group<T, 4, false, true>(v, low, sbit, G, tab);
+    store_group<T, 4>(s, v, base, sbit, G.pad);
   }
 }
 
@@ -260,21 +298,65 @@ __device__ __forceinline__ void middle_pass(typename Cx<T>::t* s, const fft::Gro
                                             const typename Cx<T>::t* tab) {
   const int n_groups = 1 << (G.log2_len - NB);
   for (int gi = threadIdx.x; gi < n_groups; gi += blockDim.x) {
-    const int base = gi << NB;
+    const int base = gi << NB;  // (NB <= pad: a group's slots are consecutive)
+    typename Cx<T>::t* p = s + fft::slot(base, G.pad);
     typename Cx<T>::t v[1 << NB];
-    load_group<T, NB>(s, v, base, 0);
+#pragma unroll
+    for (int k = 0; k < (1 << NB); ++k) v[k] = p[k];
     fft::dif_group<T, NB>(v, 0, 0, G, tab);
     T h[1 << NB];
     load_response<T, NB>(spec + base, h);
 #pragma unroll
     for (int k = 0; k < (1 << NB); ++k) v[k] = {v[k].x * h[k], v[k].y * h[k]};
     fft::dit_group<T, NB>(v, 0, 0, G, tab);
-    store_group<T, NB>(s, v, base, 0);
+#pragma unroll
+    for (int k = 0; k < (1 << NB); ++k) p[k] = v[k];
+  }
+}
+
+// The lowest two groups (bits [1, 5) and [0, 1)) together: 32 elements to a thread, the even and the odd ones.
+template <typename T>
+__device__ __forceinline__ void middle_pass_merged(typename Cx<T>::t* s, const fft::Groups& G, const T* __restrict__ spec,
+                                                   const typename Cx<T>::t* tab) {
+  using C = typename Cx<T>::t;
+  const int n_groups = 1 << (G.log2_len - 5);
+  for (int gi = threadIdx.x; gi < n_groups; gi += blockDim.x) {
+    C* p = s + fft::slot(gi << 5, 5);
+    C e[16], o[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      e[k] = p[2 * k];
+      o[k] = p[2 * k + 1];
+    }
+    fft::dif_group<T, 4>(e, 0, 1, G, tab);
+    fft::dif_group<T, 4>(o, 1, 1, G, tab);
+#pragma unroll
+    for (int k = 0; k < 16; k += 2) {
+      T h[4];
+      load_response<T, 2>(spec + (gi << 5) + 2 * k, h);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        C v[2] = {e[k + q], o[k + q]};
+        fft::dif_group<T, 1>(v, 0, 0, G, tab);
+        v[0] = {v[0].x * h[2 * q], v[0].y * h[2 * q]};
+        v[1] = {v[1].x * h[2 * q + 1], v[1].y * h[2 * q + 1]};
+        fft::dit_group<T, 1>(v, 0, 0, G, tab);
+        e[k + q] = v[0];
+        o[k + q] = v[1];
+      }
+    }
+    fft::dit_group<T, 4>(e, 0, 1, G, tab);
+    fft::dit_group<T, 4>(o, 1, 1, G, tab);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      p[2 * k] = e[k];
+      p[2 * k + 1] = o[k];
+    }
   }
 }
 
 // The top group (bits [log2 L - 4, log2 L)): optional inverse stages (the end of filter f), the pointwise op at the
-// natural-order samples, optional forward stages (the start of filter f + 1).
+// natural-order samples below L / 2 (the others are zero), optional forward stages (the start of filter f + 1).
 template <typename T>
 __device__ __forceinline__ void top_pass(typename Cx<T>::t* s, const fft::Groups& G, const MisfitArgs<T>& a,
                                          const PairCtx<T>& pc, bool inverse_first, unsigned op, bool forward_after,
@@ -284,17 +366,17 @@ __device__ __forceinline__ void top_pass(typename Cx<T>::t* s, const fft::Groups
   for (int gi = threadIdx.x; gi < n_groups; gi += blockDim.x) {
     typename Cx<T>::t v[16];
     if (inverse_first) {
-      load_group<T, 4>(s, v, gi, sbit);
-      fft::dit_group<T, 4>(v, gi, sbit, G, tab);
+      load_group<T, 4>(s, v, gi, sbit, G.pad);
+      fft::dit_group<T, 4, true>(v, gi, sbit, G, tab);
     } else {
 #pragma unroll
-      for (int k = 0; k < 16; ++k) v[k] = {(T)0, (T)0};
+      for (int k = 0; k < 8; ++k) v[k] = {(T)0, (T)0};
     }
 #pragma unroll
-    for (int k = 0; k < 16; ++k) apply_op<T>(a, pc, op, gi + (k << sbit), v[k], acc, cnt, scale);
+    for (int k = 0; k < 8; ++k) apply_op<T>(a, pc, op, gi + (k << sbit), v[k], acc, cnt, scale);
     if (forward_after) {
-      fft::dif_group<T, 4>(v, gi, sbit, G, tab);
-      store_group<T, 4>(s, v, gi, sbit);
+      fft::dif_group<T, 4, true>(v, gi, sbit, G, tab);
+      store_group<T, 4>(s, v, gi, sbit, G.pad);
     }
   }
 }
@@ -329,15 +411,9 @@ __device__ __forceinline__ void block_partials(double acc, double cnt, double* o
   }
 }
 
-template <typename T, int NB>
-__device__ __forceinline__ void middle_dispatch_(typename Cx<T>::t* s, const fft::Groups& G, const T* spec,
-                                                 const typename Cx<T>::t* tab) {
-  middle_pass<T, NB>(s, G, spec, tab);
-}
-
 // Persistent CTAs over trace pairs; dynamic shared memory = twiddle tables + L padded complex slots.
 template <typename T>
-constexpr int misfit_threads() { return sizeof(T) == 8 ? 256 : 512; }  // float64 needs twice the registers
+constexpr int misfit_threads() { return sizeof(T) == 8 ? 256 : 512; }  // at most: float64 needs twice the registers
 
 template <typename T>
 __global__ void __launch_bounds__(misfit_threads<T>()) misfit_fft_kernel(MisfitArgs<T> a, fft::Groups Gp) {
@@ -365,18 +441,21 @@ __global__ void __launch_bounds__(misfit_threads<T>()) misfit_fft_kernel(MisfitA
     top_pass<T>(s, G, a, pc, false, a.op[0], true, tab, acc, cnt, scale);
     __syncthreads();
     for (int f = 0; f < a.n_filters; ++f) {
-      for (int j = 1; j < G.count - 1; ++j) {
+      for (int j = 1; j < G.count - 1 - G.merged; ++j) {
         inner_pass<T, true>(s, G, j, tab);
         __syncthreads();
       }
-      switch (G.nb[G.count - 1]) {
-        case 1: middle_dispatch_<T, 1>(s, G, a.spec[f], tab); break;
-        case 2: middle_dispatch_<T, 2>(s, G, a.spec[f], tab); break;
-        case 3: middle_dispatch_<T, 3>(s, G, a.spec[f], tab); break;
-        default: middle_dispatch_<T, 4>(s, G, a.spec[f], tab); break;
+      if (G.merged) {
+        middle_pass_merged<T>(s, G, a.spec[f], tab);
+      } else {
+        switch (G.nb[G.count - 1]) {  // (one bit only with a group above it to merge with)
+          case 2: middle_pass<T, 2>(s, G, a.spec[f], tab); break;
+          case 3: middle_pass<T, 3>(s, G, a.spec[f], tab); break;
+          default: middle_pass<T, 4>(s, G, a.spec[f], tab); break;
+        }
       }
       __syncthreads();
-      for (int j = G.count - 2; j >= 1; --j) {
+      for (int j = G.count - 2 - G.merged; j >= 1; --j) {
         inner_pass<T, false>(s, G, j, tab);
         __syncthreads();
       }

@@ -2642,8 +2642,10 @@ int run_misfit_program(const nw_traces* t, nw::MisfitArgs<T> a, cudaStream_t s, 
   }
   const nw::fft::Groups G = nw::fft::make_groups(t->log2_len);
   const int L = 1 << t->log2_len;
-  const size_t smem = (size_t)(G.tab_len + nw::fft::slot(L - 1) + 1) * sizeof(typename nw::fft::Cx<T>::t);
-  int threads = std::min(nw::misfit_threads<T>(), std::max(32, L >> 4));
+  const size_t smem = (size_t)(G.tab_len + nw::fft::slot(L - 1, G.pad) + 1) * sizeof(typename nw::fft::Cx<T>::t);
+  // Two CTAs of 256 threads an SM up to 2^13 samples in float32 (512 threads: 1927 us where 256 take 1799, 4001
+  // samples); beyond, shared memory holds one CTA.
+  const int threads = std::min(t->log2_len <= 13 ? 256 : nw::misfit_threads<T>(), std::max(32, L >> 4));
   auto kern = nw::misfit_fft_kernel<T>;
   NW_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, sms = 0, per_sm = 0;

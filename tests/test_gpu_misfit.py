@@ -252,3 +252,23 @@ def test_filters_are_zero_phase_and_attenuate(dtype):
     low, high = torch.sin(2 * torch.pi * 2.0 * t), torch.sin(2 * torch.pi * 20.0 * t)
     y = lowpass((low + high).to(dtype), dt, f_max=6.0)
     assert float((y[100:400].double() - low[100:400]).abs().max()) < 0.05
+
+
+@pytest.mark.parametrize("dtype,n_t,n_tr", [(torch.float32, 129, 3), (torch.float64, 256, 2), (torch.float32, 4096, 37),
+                                            (torch.float32, 4097, 2)])
+def test_merged_lowest_pass_against_the_oracle(dtype, n_t, n_tr):
+    """Both ends of the trace lengths whose FFT has 4m + 1 bits (2^9 and 2^13: the lowest radix-2 stage goes with the
+    radix-16 group above it), and the first length beyond (2^14, one CTA an SM), within this file's tolerances."""
+    import misfit_oracle as mo
+
+    rng = np.random.default_rng(n_t + n_tr)
+    obs = rng.standard_normal((n_tr, n_t))
+    pred = obs + 0.5 * rng.standard_normal((n_tr, n_t))
+    mask = (rng.uniform(size=(n_tr, n_t)) > 0.1).astype(np.float64)
+    lo, go = mo.band_limited_mse(pred, obs, 0.004, 40.0, 0.3, True, mask, sensor=60.0)
+    mf = TraceMisfit(0.004, 40.0, 0.3, True, sensor_cutoff=60.0)
+    mf.prepare(_t(obs, dtype), _t(mask, dtype))
+    loss, g = mf.value_and_grad(_t(pred, dtype))
+    tl, tg = TOL[dtype]
+    assert _rel(loss, lo) < tl
+    assert rel_l2(g.cpu().numpy(), go) < tg
