@@ -590,7 +590,7 @@ def run_pat(args) -> None:
            "config": {"workload": f"pat_{n}: {n}^3 grid + 20-cell sponge ({P[0]}^3 padded), order 2, 4 instances, "
                                   f"{len(w.sensors)} sensors on one face, {op.n_steps} steps; gradient w.r.t. p0 and c; "
                                   f"checkpointed with {args.snapshot} snapshots",
-                      "method": "plain (per-step launches)",
+                      "method": "plain (per problem)",
                       "l2": "working set (4 x {0:.0f} MB per level) far above L2".format(cells * 16 / 1e6)},
            "gcell_updates_per_s": useful / (ms * 1e-3) / 1e9,
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -1221,7 +1221,7 @@ def main() -> None:
                "vs_baseline": None, "dtype": "f32",
                "data": "synthetic (seeded layered model; observed data from a smoothed model)",
                "config": {**workload_desc(w, storage, absorbing),
-                          "method": f"plain (per-step launches replayed from one CUDA graph, {storage})",
+                          "method": f"plain (sweeps replayed from one CUDA graph, {storage})",
                           "tuning": list(op.tuning) if getattr(op, "tuning", None) else "library defaults",
                           "parallelism": f"shots sharded over {world} GPU(s), fp64 gradient and loss all-reduce"},
                "gcell_updates_per_s": gcells, "roofline": roofline, "cpu_baseline": cpu,

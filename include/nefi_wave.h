@@ -265,6 +265,11 @@ int nw_initial_state(const nw_grid* g, const int32_t* n_abs, const nw_medium* m,
  * n in [n_begin, n_end) go to traces (n_shots, n_rec, n_t), and of level n_end when it is the last
  * step; with checkpointing, snapshots of every segment start in [n_begin, n_end) are encoded.
  * On entry ring levels n_begin-1 and n_begin must be in place. `tune` may be NULL.
+ * A 2-D sweep whose state fits the chip runs as one launch for all its steps, a thread-block cluster per
+ * shot, where that is the quicker way (depth 0 or 1); fields, traces and stored levels are bitwise those of one
+ * launch per step. It leaves the last two levels in the ring, not the intermediate ones. CTAs of a cluster wait
+ * for one another's edge rows; a wait that gives up sets the status word (NW_ERR_TIMEOUT, read by nw_status)
+ * and puts a NaN into the field.
  * With the PML and an interior box of at least one tile, each step forks its layer kernel onto a
  * second stream of the calling thread and joins it back into `stream` (also in nw_adjoint and the
  * batched sweeps); the first such call on a thread and device creates that stream and two events,
@@ -285,7 +290,8 @@ int nw_forward(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, co
  *    needed by the initial-value operator.
  * The steps advance q = c2dt2 * mu, which obeys the forward recursion with the source replaced
  * by c2dt2 * R^T g_n; `work` holds three q levels (3 * n_shots fields; 7 * n_shots with a PML, whose
- * adjoint also carries the face cotangents of psi, 2 axes x 2 levels). Uses the history or
+ * adjoint also carries the face cotangents of psi, 2 axes x 2 levels); a sweep of many steps per launch (see
+ * nw_forward) keeps the per-shot sums in the third one. Uses the history or
  * recomputes segments from the snapshots in `st`. This is the discrete adjoint torch.autograd
  * derives from nefi/physics/wave.py:529-552 and nefi/physics/timestep.py:151-169.
  */
@@ -367,8 +373,9 @@ uint64_t nw_launch_count(void);
 
 /*
  * Batched FWI gradients: many independent 2-D problems (grids of different size, shot counts and
- * step counts, one dtype and stencil order) advanced together, one launch per time step for the
- * whole batch. This has no single counterpart in the reference, whose operators cannot be batched
+ * step counts, one dtype and stencil order) advanced together: those whose sweeps take many steps per
+ * launch alone (see nw_forward) do so here, side by side on up to eight streams of the calling thread, the
+ * others by one launch per time step for all of them. This has no single counterpart in the reference, whose operators cannot be batched
  * (nefi/solve/batched.py:68-77); each problem's traces and gradient are those nw_forward /
  * nw_adjoint give it alone with the same tuning and snapshots (bitwise).
  *
@@ -403,7 +410,8 @@ int nw_batch_prepare(const nw_batch_problem* problems, int32_t n_problems, const
 
 /*
  * Forward sweep of the whole batch from p^-1 = p^0 = 0: traces of every problem, and the
- * snapshots of every segment start. One kernel per global step over the problems still running
+ * snapshots of every segment start. For the problems advanced together one kernel per global step over those
+ * still running
  * (a PML problem's interior box; its layer cells and receivers take launches of their own), plus
  * the snapshot encodes and each problem's final receiver sample. Asynchronous; no host
  * synchronisation, so a caller may capture it in a CUDA graph.
