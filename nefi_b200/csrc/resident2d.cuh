@@ -1073,11 +1073,12 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
           a.traces[(long long)s * a.n_rec * a.n_t + l_id[e] + j] = v;
         };
         if (sampled && id < 32) {
-          const int n_edge = count[1];
-          if (rec && n_edge > 0) {
-            if (has_dn) wait_halo(1, m);
-            for (int e = id; e < n_edge; e += 32) sample(a.cap_list - 1 - e);
-          }
+          const int n_edge = rec ? count[1] : 0;
+          // The wait is not for the samples alone: the piece below counts towards the phase of step m + 1, which
+          // shares its mbarrier with that of m - 1, and only the rows this waits for say that the CTA below has
+          // seen m - 1 complete.
+          if (has_dn && (n_edge > 0 || !last)) wait_halo(1, m);
+          for (int e = id; e < n_edge; e += 32) sample(a.cap_list - 1 - e);
           __syncwarp();
           if (id == 0 && has_dn && !last)
             send_bytes(smem_addr(buf) + dn_off + a.nv * 16 + ((m + 1) % NL) * (unsigned)(BS * (int)sizeof(T)),
