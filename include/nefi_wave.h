@@ -83,8 +83,12 @@ int nw_grid_layout(nw_grid* g);
 /*
  * Launch shape of the 2-D step kernels, forward and adjoint separately: a CTA owns a tile of
  * 8*rx rows by 32*vz columns and loops over shots_per_cta shots. Zero fields take the library's
- * defaults. 3-D grids ignore it.
+ * defaults. 3-D grids ignore it. The shapes are those of the launches of one step (or two, see depth);
+ * a sweep that takes all its steps in one launch (see nw_forward; nw_sweep_route tells) has none of them,
+ * only adj_shots_per_cta still says which shots share an accumulator. `flags` keeps a direction to the
+ * launches of one step.
  */
+enum { NW_TUNE_ONE_STEP_FORWARD = 1, NW_TUNE_ONE_STEP_ADJOINT = 2 };
 typedef struct nw_tuning {
   int32_t vz;                /* forward: columns per thread, 2 or 4 (float32), 2 (float64) */
   int32_t rx;                /* forward: rows per thread, 2, 4 or 8 */
@@ -97,7 +101,8 @@ typedef struct nw_tuning {
                                 give bitwise the fields of one. With depth 2 the forward tile of
                                 nw_tile_shape is the core a launch stores: (8*rx - 2*radius) rows by
                                 (32*vz - 2*(16 / element size)) columns */
-  int32_t reserved;
+  int32_t flags;             /* NW_TUNE_ONE_STEP_* combined, 0: the quicker way; a value that is no
+                                combination of them counts as 0 */
 } nw_tuning;
 
 /*
@@ -298,6 +303,15 @@ int nw_forward(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, co
 int nw_adjoint(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
                const nw_storage* st, const nw_tuning* tune, const void* grad_traces, void* work,
                void* grad_acc, void* lambda0, void* mu1, void* stream);
+
+/*
+ * How the forward (adjoint = 0) or adjoint (1) sweep of this problem runs on the current device:
+ * route = {CTAs that hold a shot, grid rows a thread steps} of a sweep with all its steps in one launch,
+ * or {0, 0} for launches of one or two steps. Reads the grid, m->pml_core and the counts of `a` and `t`;
+ * launches nothing.
+ */
+int nw_sweep_route(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
+                   const nw_tuning* tune, int32_t adjoint, int32_t* route);
 
 /*
  * The adjoint run of nw_adjoint for the initial state alone (lambda0 and mu1, both required): without the

@@ -21,6 +21,7 @@ NW_ABS_NONE, NW_ABS_SPONGE, NW_ABS_CERJAN, NW_ABS_PML = 0, 1, 2, 3
 NW_SNAP_EXACT, NW_SNAP_F16, NW_SNAP_BF16 = 0, 1, 2
 NW_OK, NW_ERR_ARG, NW_ERR_CUDA, NW_ERR_UNSUPPORTED, NW_ERR_NONFINITE, NW_ERR_TIMEOUT = range(6)
 NW_SNAP_BLOCK = 32
+ONE_STEP_FORWARD, ONE_STEP_ADJOINT = 1, 2  # Tuning.flags
 
 NW_SNAP_I16 = 3
 NW_SNAP_D16 = 4
@@ -41,7 +42,7 @@ class Grid(C.Structure):
 class Tuning(C.Structure):
     _fields_ = [("vz", C.c_int32), ("rx", C.c_int32), ("shots_per_cta", C.c_int32),
                 ("adj_vz", C.c_int32), ("adj_rx", C.c_int32), ("adj_shots_per_cta", C.c_int32),
-                ("depth", C.c_int32), ("reserved", C.c_int32)]
+                ("depth", C.c_int32), ("flags", C.c_int32)]
 
 
 class Acquisition(C.Structure):
@@ -110,6 +111,7 @@ _SIGNATURES = {
                              C.c_int32, C.c_int32, VP, VP]),
     "nw_adjoint": (C.c_int, [P(Grid), P(Medium), P(Acquisition), P(Time), P(Storage), P(Tuning), VP,
                              VP, VP, VP, VP, VP]),
+    "nw_sweep_route": (C.c_int, [P(Grid), P(Medium), P(Acquisition), P(Time), P(Tuning), C.c_int32, P(C.c_int32)]),
     "nw_adjoint_initial": (C.c_int, [P(Grid), P(Medium), P(Acquisition), P(Time), P(Tuning), VP, VP, VP, VP, VP]),
     "nw_reduce_grad_c": (C.c_int, [P(Grid), VP, VP, C.c_double, C.c_int32, VP, C.c_int32, VP, VP]),
     "nw_initial_state_adjoint": (C.c_int, [P(Grid), VP, P(Medium), P(Time), C.c_int32, VP, VP, VP,

@@ -282,6 +282,7 @@ struct TileCfg {  // one 2-D step kernel's tile: 8*rx rows by 32*vz columns, spc
 };
 struct Tune {
   TileCfg fwd, adj;
+  bool fwd_one = false, adj_one = false;  // one step per launch asked for (NW_TUNE_ONE_STEP_*)
 };
 
 int check_tile(const nw_grid* g, const TileCfg& c, const char* which) {
@@ -310,6 +311,10 @@ int resolve_tune(const nw_grid* g, const nw_tuning* t, Tune* out) {
   // two forward steps per launch: 2-D grids without a PML (whose steps run a layer kernel beside the box)
   r.fwd.depth = (t && t->depth == 2 && g->ndim == 2 && g->absorbing != NW_ABS_PML) ? 2 : 1;
   if (t && (t->depth < 0 || t->depth > 2)) return fail(NW_ERR_ARG, "tuning.depth must be 0, 1 or 2");
+  if (t && (t->flags & ~(NW_TUNE_ONE_STEP_FORWARD | NW_TUNE_ONE_STEP_ADJOINT)) == 0) {
+    r.fwd_one = (t->flags & NW_TUNE_ONE_STEP_FORWARD) != 0;
+    r.adj_one = (t->flags & NW_TUNE_ONE_STEP_ADJOINT) != 0;
+  }
   r.fwd.r = r.adj.r = g->radius;
   r.fwd.hl = r.adj.hl = g->dtype == NW_F64 ? 2 : 4;
   *out = r;
@@ -643,12 +648,12 @@ int launch_resident_v(const nw::KGrid<T>& kg, const nw::Resident<T>& a, const Re
 }
 
 // The plan of a forward or adjoint resident sweep of these shots (ok = false: the grid does not fit a
-// cluster's shared memory and registers, or has three dimensions).
+// cluster's shared memory and registers, has three dimensions, or the tuning asks for one step per launch).
 template <typename T, bool ADJ>
-int resident_for(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t, ResidentPlan* p,
-                 bool crowded = false, int n_imposed = 0) {
+int resident_for(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t, const Tune& tu,
+                 ResidentPlan* p, bool crowded = false, int n_imposed = 0) {
   *p = ResidentPlan();
-  if (g->ndim != 2) return NW_OK;
+  if (g->ndim != 2 || (ADJ ? tu.adj_one : tu.fwd_one)) return NW_OK;
   if ((long long)a->n_rec * t->n_t > INT_MAX) return NW_OK;
   auto plan = [&](bool c) {
     return g->radius == 1 ? resident_plan<T, 1, ADJ>(g, m, a->n_shots, n_imposed ? 0 : a->n_rec, a->n_cells, n_imposed, c, p)
@@ -1151,7 +1156,7 @@ int forward_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
   const bool pairs = g->ndim == 2 && tu.fwd.depth == 2 && L.levels == 4;
   ResidentPlan res;
   if (!pairs) {
-    const int rc = resident_for<T, false>(g, m, a, t, &res, crowded);
+    const int rc = resident_for<T, false>(g, m, a, t, tu, &res, crowded);
     if (rc) return rc;
   }
   // a resident sweep writes exact snapshots itself (their ghost cells stay zero)
@@ -1231,8 +1236,8 @@ int adjoint_impl(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
   const bool pairs = g->ndim == 2 && tu.fwd.depth == 2 && L.levels == 4;
   ResidentPlan res, fres;  // the adjoint's and the recompute's resident sweeps
   {
-    int rc = resident_for<T, true>(g, m, a, t, &res, crowded);
-    if (!rc && ckpt && !pairs) rc = resident_for<T, false>(g, m, a, t, &fres, crowded);
+    int rc = resident_for<T, true>(g, m, a, t, tu, &res, crowded);
+    if (!rc && ckpt && !pairs) rc = resident_for<T, false>(g, m, a, t, tu, &fres, crowded);
     if (rc) return rc;
   }
   // forward steps [k0, k1) of a recompute or an advance; Lap p^k into seg + (k - k0) levels if seg
@@ -1715,6 +1720,26 @@ int nw_adjoint_initial(const nw_grid* g, const nw_medium* m, const nw_acquisitio
                               (double*)mu1, (cudaStream_t)stream);
 }
 
+int nw_sweep_route(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
+                   const nw_tuning* tune, int32_t adjoint, int32_t* route) {
+  int rc = check_grid(g);
+  if (rc) return rc;
+  if (!m || !a || !t || !route) return fail(NW_ERR_ARG, "NULL argument");
+  Tune tu;
+  rc = resolve_tune(g, tune, &tu);
+  if (rc) return rc;
+  ResidentPlan p;
+  if (adjoint || tu.fwd.depth != 2) {
+    if (g->dtype == NW_F32)
+      rc = adjoint ? resident_for<float, true>(g, m, a, t, tu, &p) : resident_for<float, false>(g, m, a, t, tu, &p);
+    else
+      rc = adjoint ? resident_for<double, true>(g, m, a, t, tu, &p) : resident_for<double, false>(g, m, a, t, tu, &p);
+  }
+  route[0] = p.ok ? p.cluster : 0;
+  route[1] = p.ok ? p.rx : 0;
+  return rc;
+}
+
 int nw_reduce_grad_c(const nw_grid* g, const int32_t* n_abs, const void* c, double dt2,
                      int32_t n_acc, const void* grad_acc, int32_t accumulate, double* grad_c,
                      void* stream) {
@@ -1939,21 +1964,23 @@ int check_batch(const nw_batch_problem* P, int n, const Tune& tu) {
   return NW_OK;
 }
 
+// Whether problem q takes resident sweeps: it then runs apart.
+template <typename T>
+int batch_solo(const nw_batch_problem& q, const Tune& tu, bool* solo) {
+  ResidentPlan f, a;
+  int rc = resident_for<T, false>(&q.grid, &q.medium, &q.acq, &q.time, tu, &f);
+  if (!rc) rc = resident_for<T, true>(&q.grid, &q.medium, &q.acq, &q.time, tu, &a);
+  *solo = f.ok || a.ok;
+  return rc;
+}
+
 // The tiles a batched launch steps for problem q: the whole grid, or with a PML the interior box
 // (the layer goes through the PML kernel in launches of its own). The box depends on T only through
 // its 16-byte column alignment, which the batch's dtype fixes.
 template <typename T>
-int batch_solo(const nw_batch_problem& q, bool* solo) {  // whether q takes resident sweeps: it then runs apart
-  ResidentPlan f, a;
-  int rc = resident_for<T, false>(&q.grid, &q.medium, &q.acq, &q.time, &f);
-  if (!rc) rc = resident_for<T, true>(&q.grid, &q.medium, &q.acq, &q.time, &a);
-  *solo = f.ok || a.ok;
-  return rc;
-}
-template <typename T>
-dim3 batch_grid(const nw_batch_problem& q, const TileCfg& c) {
+dim3 batch_grid(const nw_batch_problem& q, const Tune& tu, const TileCfg& c) {
   bool solo = false;
-  if (batch_solo<T>(q, &solo) || solo) return dim3(0, 0, 0);
+  if (batch_solo<T>(q, tu, &solo) || solo) return dim3(0, 0, 0);
   if (q.grid.absorbing != NW_ABS_PML) return c.grid(&q.grid, q.acq.n_shots);
   nw::PmlStep<T> st = {};
   if (pml_tiled_box<T>(&q.grid, &q.medium, c, st) || st.kx1 == st.kx0) return dim3(0, 0, 0);
@@ -2026,7 +2053,7 @@ int batch_prepare_impl(const nw_batch_problem* P, int n, const Tune& tu, void* t
         B.adj.n_rec = a->n_rec;
       }
     }
-    const dim3 fg = batch_grid<T>(q, tu.fwd), ag = batch_grid<T>(q, tu.adj);
+    const dim3 fg = batch_grid<T>(q, tu, tu.fwd), ag = batch_grid<T>(q, tu, tu.adj);
     B.ftx = (int)fg.y;
     B.atx = (int)ag.y;
     fcta[p] = (int)fsum;
@@ -2065,11 +2092,11 @@ int batch_solos(const nw_batch_problem* P, const std::vector<char>& solo, cudaSt
   });
 }
 template <typename T>
-int batch_solo_flags(const nw_batch_problem* P, int n, std::vector<char>* solo) {
+int batch_solo_flags(const nw_batch_problem* P, int n, const Tune& tu, std::vector<char>* solo) {
   solo->assign(n, 0);
   for (int p = 0; p < n; ++p) {
     bool f = false;
-    const int rc = batch_solo<T>(P[p], &f);
+    const int rc = batch_solo<T>(P[p], tu, &f);
     if (rc) return rc;
     (*solo)[p] = f;
   }
@@ -2129,10 +2156,10 @@ int launch_adj_batch(const void* table, int n, int n_active, int n_ctas, int ste
 
 // Host copy of the CTA offsets: cta[p] = CTAs of the problems before p.
 template <typename T>
-std::vector<int> batch_ctas(const nw_batch_problem* P, int n, const TileCfg& c) {
+std::vector<int> batch_ctas(const nw_batch_problem* P, int n, const Tune& tu, const TileCfg& c) {
   std::vector<int> cta(n + 1, 0);
   for (int p = 0; p < n; ++p) {
-    const dim3 gr = batch_grid<T>(P[p], c);
+    const dim3 gr = batch_grid<T>(P[p], tu, c);
     cta[p + 1] = cta[p] + (int)(gr.x * gr.y * gr.z);
   }
   return cta;
@@ -2234,14 +2261,14 @@ void batch_pml_faces(const nw_batch_problem& q, int k, T* out[2]) {
 template <typename T>
 int batch_forward_impl(const nw_batch_problem* P, int n, const Tune& tu, const void* table, cudaStream_t s) {
   const int K = P[0].storage.segment, Nmax = P[0].time.n_steps, R = P[0].grid.radius;
-  const std::vector<int> cta = batch_ctas<T>(P, n, tu.fwd);
+  const std::vector<int> cta = batch_ctas<T>(P, n, tu, tu.fwd);
   for (int p = 0; p < n; ++p) {  // p^-1 = p^0 = 0 (FWI), and the PML's face fields
     const size_t lvl = (size_t)P[p].acq.n_shots * P[p].grid.field_elems * sizeof(T);
     NW_CUDA(cudaMemsetAsync(P[p].storage.ring, 0, 3 * lvl, s));
     if (P[p].grid.absorbing == NW_ABS_PML) NW_CUDA(cudaMemsetAsync(P[p].storage.pml_psi, 0, 4 * lvl, s));
   }
   std::vector<char> solo;
-  int rc0 = batch_solo_flags<T>(P, n, &solo);
+  int rc0 = batch_solo_flags<T>(P, n, tu, &solo);
   if (rc0) return rc0;
   auto tiled_pml = [&](int p) { return P[p].grid.absorbing == NW_ABS_PML && !solo[p]; };
   auto rest = [&]() -> int {  // the others, together, a step per launch
@@ -2298,9 +2325,9 @@ int batch_forward_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
 template <typename T>
 int batch_adjoint_impl(const nw_batch_problem* P, int n, const Tune& tu, const void* table, cudaStream_t s) {
   const int K = P[0].storage.segment, Nmax = P[0].time.n_steps, R = P[0].grid.radius;
-  const std::vector<int> fcta = batch_ctas<T>(P, n, tu.fwd), acta = batch_ctas<T>(P, n, tu.adj);
+  const std::vector<int> fcta = batch_ctas<T>(P, n, tu, tu.fwd), acta = batch_ctas<T>(P, n, tu, tu.adj);
   std::vector<char> solo;
-  int rc0 = batch_solo_flags<T>(P, n, &solo);
+  int rc0 = batch_solo_flags<T>(P, n, tu, &solo);
   if (rc0) return rc0;
   auto tiled_pml = [&](int p) { return P[p].grid.absorbing == NW_ABS_PML && !solo[p]; };
   for (int p = 0; p < n; ++p) {
@@ -2464,7 +2491,7 @@ int time_reversal_impl(const nw_grid* g, const nw_medium* m, const nw_acquisitio
   int rc = impose(0);
   if (rc) return rc;
   ResidentPlan res;
-  if (tu.fwd.depth != 2) rc = resident_for<T, false>(g, m, a, t, &res, false, n_cells);
+  if (tu.fwd.depth != 2) rc = resident_for<T, false>(g, m, a, t, tu, &res, false, n_cells);
   if (rc) return rc;
   if (res.ok && N >= kResidentSteps)  // the steps and the later levels' conditions in one launch
     return resident_forward<T>(g, kg, m, a, t, res, L.at(-1), L.at(0), L.at(N - 1), L.at(N), 0, N, nullptr, nullptr,

@@ -176,11 +176,13 @@ class DevicePlan:
         self.set_tuning(*(getattr(op, "tuning", None) or ()))
 
     def set_tuning(self, vz: int = 0, rx: int = 0, shots_per_cta: int = 0, adj_vz: int = 0, adj_rx: int = 0,
-                   adj_shots_per_cta: int = 0, depth: int = 0) -> None:
+                   adj_shots_per_cta: int = 0, depth: int = 0, flags: int = 0) -> None:
         """Choose the 2-D launch shapes (0 = library default) and the forward steps per launch
-        (``depth`` 2: two, on 2-D grids without a PML), and build the per-tile tables."""
+        (``depth`` 2: two, on 2-D grids without a PML), and build the per-tile tables. The shapes are those of
+        launches of one step or two: a sweep that takes all its steps in one launch (``sweep_route``) has none;
+        ``flags`` (``_lib.ONE_STEP_FORWARD``, ``_lib.ONE_STEP_ADJOINT``) keeps a direction to launches of one."""
         t = _lib.Tuning(int(vz), int(rx), int(shots_per_cta), int(adj_vz), int(adj_rx), int(adj_shots_per_cta),
-                        int(depth))
+                        int(depth), int(flags))
         shape = (C.c_int32 * 4)()
         _lib.check(_lib.load().nw_tile_shape(C.byref(self.g), C.byref(t), shape))
         self.tuning = t
@@ -259,6 +261,17 @@ class DevicePlan:
         if x1 - x0 < tx or z1 - z0 < tz:
             return None
         return x0, x1, z0, z1
+
+    def sweep_route(self, n_shots: int, adjoint: bool = False) -> tuple[int, int]:
+        """``(CTAs that hold a shot, grid rows a thread steps)`` of the forward or adjoint sweep with all its
+        steps in one launch, ``(0, 0)`` when it takes launches of one step or two."""
+        m, route = _lib.Medium(), (C.c_int32 * 2)()
+        for k in range(4 if self.pml is not None else 0):
+            m.pml_core[k] = self.pml["core"][k]
+        with torch.cuda.device(self.device):
+            _lib.check(_lib.load().nw_sweep_route(C.byref(self.g), C.byref(m), C.byref(self.acquisition(n_shots)),
+                                                  C.byref(self.time), C.byref(self.tuning), int(adjoint), route))
+        return route[0], route[1]
 
     def n_acc(self, n_shots: int) -> int:
         """Gradient accumulator fields (plan dtype) the adjoint sweep fills for ``n_shots`` shots."""
