@@ -88,7 +88,12 @@ int nw_grid_layout(nw_grid* g);
  * only adj_shots_per_cta still says which shots share an accumulator. `flags` keeps a direction to the
  * launches of one step.
  */
-enum { NW_TUNE_ONE_STEP_FORWARD = 1, NW_TUNE_ONE_STEP_ADJOINT = 2 };
+enum {
+  NW_TUNE_ONE_STEP_FORWARD = 1,
+  NW_TUNE_ONE_STEP_ADJOINT = 2,
+  NW_TUNE_MUTE = 4 /* for tests of the failure report: in a sweep with all its steps in one launch the first of a
+                      shot's CTAs sends no rows, so that the waits for them run out */
+};
 typedef struct nw_tuning {
   int32_t vz;                /* forward: columns per thread, 2 or 4 (float32), 2 (float64) */
   int32_t rx;                /* forward: rows per thread, 2, 4 or 8 */
@@ -101,7 +106,7 @@ typedef struct nw_tuning {
                                 give bitwise the fields of one. With depth 2 the forward tile of
                                 nw_tile_shape is the core a launch stores: (8*rx - 2*radius) rows by
                                 (32*vz - 2*(16 / element size)) columns */
-  int32_t flags;             /* NW_TUNE_ONE_STEP_* combined, 0: the quicker way; a value that is no
+  int32_t flags;             /* NW_TUNE_* combined, 0: the quicker way; a value that is no
                                 combination of them counts as 0 */
 } nw_tuning;
 
@@ -273,8 +278,9 @@ int nw_initial_state(const nw_grid* g, const int32_t* n_abs, const nw_medium* m,
  * A 2-D sweep whose state fits the chip runs as one launch for all its steps, a thread-block cluster per
  * shot, where that is the quicker way (depth 0 or 1); fields, traces and stored levels are bitwise those of one
  * launch per step. It leaves the last two levels in the ring, not the intermediate ones. CTAs of a cluster wait
- * for one another's edge rows; a wait that gives up sets the status word (NW_ERR_TIMEOUT, read by nw_status)
- * and puts a NaN into the field.
+ * for one another's edge rows, 0.2 seconds at most (they come within microseconds). If such a wait gives up, the
+ * sweep runs to its end, all that it writes for the shot is NaN, and the next call that runs a sweep on the device,
+ * nw_reported or nw_status returns NW_ERR_TIMEOUT, once.
  * With the PML and an interior box of at least one tile, each step forks its layer kernel onto a
  * second stream of the calling thread and joins it back into `stream` (also in nw_adjoint and the
  * batched sweeps); the first such call on a thread and device creates that stream and two events,
@@ -528,12 +534,15 @@ int nw_misfit(const nw_traces* t, const void* pred, const void* obs, const void*
               const void* loss_response, double* state, void* grad, void* stream);
 
 /*
- * Synchronises `stream`, then returns and clears the device status word that kernels set on a
- * detected failure (a non-finite snapshot block: NW_ERR_NONFINITE). The word is shared by all
+ * Synchronises `stream`, then returns and clears the device status that kernels set on a
+ * detected failure (a non-finite snapshot block: NW_ERR_NONFINITE; a wait that gave up: NW_ERR_TIMEOUT). The word is shared by all
  * streams of the current device. NEFI raises OperatorError/SolverError for such failures
  * (nefi/physics/wave.py:561-569, nefi/errors.py:22-27).
  */
 int nw_status(void* stream);
+/* NW_ERR_TIMEOUT, once, if a sweep that ran on the current device gave up a wait (see nw_forward), else NW_OK.
+ * Does not synchronise: it sees what has been reported so far. The calls that run sweeps ask first. */
+int nw_reported(void);
 
 /* Message of the calling thread's last error ("" if none). Host only. */
 const char* nw_last_error(void);

@@ -21,7 +21,7 @@ NW_ABS_NONE, NW_ABS_SPONGE, NW_ABS_CERJAN, NW_ABS_PML = 0, 1, 2, 3
 NW_SNAP_EXACT, NW_SNAP_F16, NW_SNAP_BF16 = 0, 1, 2
 NW_OK, NW_ERR_ARG, NW_ERR_CUDA, NW_ERR_UNSUPPORTED, NW_ERR_NONFINITE, NW_ERR_TIMEOUT = range(6)
 NW_SNAP_BLOCK = 32
-ONE_STEP_FORWARD, ONE_STEP_ADJOINT = 1, 2  # Tuning.flags
+ONE_STEP_FORWARD, ONE_STEP_ADJOINT, MUTE = 1, 2, 4  # Tuning.flags
 
 NW_SNAP_I16 = 3
 NW_SNAP_D16 = 4
@@ -118,6 +118,7 @@ _SIGNATURES = {
                                            VP, VP, C.c_int32, VP]),
     "nw_sample": (C.c_int, [P(Grid), P(Acquisition), C.c_int32, VP, C.c_int32, VP, VP]),
     "nw_status": (C.c_int, [VP]),
+    "nw_reported": (C.c_int, []),
     "nw_zero_ghosts": (C.c_int, [P(Grid), VP, C.c_int64, VP]),
     "nw_adjoint_grad_c_noalloc": (C.c_int, [P(Grid), VP, P(Medium), P(Acquisition), P(Time), P(Storage),
                                             P(Tuning), VP, C.c_double, VP, VP, VP]),

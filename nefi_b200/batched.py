@@ -176,6 +176,7 @@ class BatchedFWI:
         float64 (the tensors are reused by the next call: clone to keep them)."""
         self._load(cs, observed)
         if self._graph is not None:
+            _lib.check(_lib.load().nw_reported())
             self._graph.replay()
         else:
             self._step()
@@ -184,8 +185,10 @@ class BatchedFWI:
 
     @_lib.on_device
     def check_snapshots(self) -> None:
-        """Synchronise and raise if a 16-bit snapshot block held a non-finite value."""
+        """Synchronise and raise if a 16-bit snapshot block held a non-finite value (exact snapshots have no
+        such check); raise if a sweep has reported that a wait inside it gave up."""
         if self.snapshot == "exact":
+            _lib.check(_lib.load().nw_reported())
             return
         rc = _lib.load().nw_status(_lib.stream_handle(self.device))
         if rc == _lib.NW_ERR_NONFINITE:

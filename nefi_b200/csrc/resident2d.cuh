@@ -12,8 +12,11 @@
 // waits for its two neighbours only, and no cluster-wide barrier (with the fence it carries) is paid per
 // step. p^{n+1} arrives in the halo rows that held p^{n-1}: the neighbour sends it once all of this CTA's
 // edge rows of p^n have reached it, and every warp that reads a halo row of p^{n-1} sends its piece of an edge
-// row of p^n after that read, so nobody reads the rows any more. Waits are bounded: one that gives up sets the
-// device status word and puts a NaN into the field, and the kernel runs on without waiting.
+// row of p^n after that read, so nobody reads the rows any more.
+//
+// Waits are bounded. A thread that gives one up waits and sends no more, its CTA arms no further phase, and the
+// neighbours' waits run out in turn. The kernel runs to its end, writes NaN for all results of a shot of whose CTAs one
+// gave up, and tells the host (Resident::report).
 //
 // Threads: a row has NV vectors of VZ = 16 / sizeof(T) columns, a slab S strips of rows; a thread steps one
 // vector of one strip, marching over at most RX rows with a (2R+1)-row register window. The vectors that hold
@@ -99,6 +102,8 @@ struct Resident {
   const T* __restrict__ imposed_tr;
   int n_imposed;
   int n_rec, n_t, n_cells;
+  int mute;        // 1: the first CTA of a shot sends nothing (to test what follows)
+  int* report;     // host memory: set to NW_ERR_TIMEOUT when a wait gave up
   int cap_list;  // receivers (forward) or touched cells (adjoint) the shared tables hold: at least all of them
   int cap_ent;   // adjoint: the table entries they hold
 };
@@ -163,9 +168,10 @@ __device__ __forceinline__ void mbar_init(unsigned bar) {
 __device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Waits for the phase of parity `par`; false if it did not complete within the limit (seconds).
+// Waits for the phase of parity `par`; false if it did not complete within 2^17 tries, 0.2 s. (A try that fails takes
+// 1.5 us, measured. A limit that is no constant, or a look at the clock, cost a step of 128^2 or 256^2 0.2 to 0.6 us.)
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned par) {
-  for (int i = 0; i < (1 << 22); ++i) {
+  for (int i = 0; i < (1 << 17); ++i) {
     unsigned done;
     asm volatile(
         "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
@@ -222,6 +228,33 @@ __device__ __forceinline__ int2 count_below(const int64_t* idx, int n, long long
   return total;
 }
 
+// The report to the host, and NaN in the place of all that a CTA of shot s has written: in the levels, the gradient sums, Lap p and the snapshots the
+// strip of `nr` rows whose first vector (of column zc) is at `cell`, and all samples. Copies that nobody waited for then
+// have had a millisecond to land. (Not inlined: it would cost the time loops registers.)
+template <typename T, int VZ, bool ADJ>
+__device__ __noinline__ void mark_lost(const Resident<T>& a, int s, long long cell, int nr, int dld, int zc, int n1) {
+  const long long t0 = clock64();
+  *(volatile int*)a.report = 5;  // NW_ERR_TIMEOUT
+  T bad[VZ];
+  for (int v = 0; v < VZ; ++v) bad[v] = T(NAN);
+  for (int k = 0; k < nr; ++k, cell += dld) {
+    T* fields[3] = {a.out_cur, a.out_prev, ADJ ? a.acc : nullptr};
+    for (T* f : fields)
+      if (f) store_row<T, VZ>(f + cell, bad, zc, n1);
+    for (int n = a.n_first; !ADJ && n < a.n_first + a.count; ++n) {
+      if (a.lap_out) store_row<T, VZ>(a.lap_out + (n - a.n_first) * a.level + cell, bad, zc, n1);
+      if (a.snap && n % a.segment == 0)
+        for (int l = 0; l < 2; ++l)
+          store_row<T, VZ>(a.snap + (long long)(n / a.segment) * a.snap_stride + l * a.level + cell, bad, zc, n1);
+    }
+  }
+  if (!ADJ && a.traces)
+    for (int n = a.n_first; n < a.n_first + a.count; ++n)
+      for (int e = threadIdx.x; n % a.substeps == 0 && e < a.n_rec; e += blockDim.x)
+        a.traces[((long long)s * a.n_rec + e) * a.n_t + n / a.substeps] = T(NAN);
+  for (int i = 0; i < 10000 && clock64() - t0 < 2000000; ++i) __nanosleep(1000);
+}
+
 // IMP: the forward of a time reversal, which imposes cells after each step (apart: it costs registers).
 template <typename T, int R, int RX, bool ADJ, bool PML, bool IMP>
 __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __grid_constant__ KGrid<T> g, const __grid_constant__ Resident<T> a) {
@@ -270,9 +303,11 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
 #pragma unroll
   for (int u = 0; u < VZ; ++u) zero[u] = T(0);
   for (int i = tid; i < NL * (BS / VZ); i += nthr) vstore<T, VZ>(buf - VZ + i * VZ, zero);
+  __shared__ int gave_up, lost_sh;  // a wait of this CTA, of one of the shot's CTAs, gave up
   if (tid == 0) {
     for (int i = 0; i < 4; ++i) mbar_init(mbar_a + 8 * i);
     count[0] = 0;
+    gave_up = lost_sh = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
@@ -550,13 +585,15 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
     if (work) vload<T, VZ>(a.f_in[0] + so + cell0 + (long long)nr * ld, f_end);
   }
   const bool need_up = work && has_up && ra - R < 0, need_dn = work && has_dn && rb + R > rows;
-  bool dead = false;  // a wait gave up: run on without waiting, the field marked with a NaN
+  bool dead = false;  // a wait of this thread gave up: it runs on without waiting or sending
+  // (The results are marked at the end: NaN put into the rows or registers here cost a step of 128^2 3 % and more.)
+  auto give_up = [&]() {
+    dead = true;
+    *(volatile int*)&gave_up = 1;
+  };
   auto wait_halo = [&](int side, int m) {
     if (m == 0 || dead) return;
-    if (!mbar_wait(mbar_a + 16 * side + 8 * (m & 1), ((m - 1) >> 1) & 1)) {
-      dead = true;
-      atomicExch(&g_status, 5);  // NW_ERR_TIMEOUT
-    }
+    if (!mbar_wait(mbar_a + 16 * side + 8 * (m & 1), ((m - 1) >> 1) & 1)) give_up();
   };
   T lpb[PF][VZ];  // Lap p of the next rows (adjoint)
   auto lap_of = [&](int n) -> const T* {  // this march's Lap p of step n
@@ -583,7 +620,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
     const unsigned mask = (seg_end == 32 ? ~0u : (1u << seg_end) - 1) & ~((1u << seg_first) - 1);
     fence_async();
     __syncwarp(mask);
-    if (((int)threadIdx.x & 31) != seg_first) return;
+    if (((int)threadIdx.x & 31) != seg_first || dead) return;
     const int row_b = pitch * (int)sizeof(T);
     const unsigned own = smem_addr(buf) + zc * (unsigned)sizeof(T) + level * (unsigned)(BS * (int)sizeof(T));
     const unsigned to = own + (side ? dn_off + (R - rows) * row_b : up_off + (R + X0 - a.slab[rank - 1]) * row_b);
@@ -598,6 +635,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
   // It releases the bottom halo rows only after the receivers that read them are sampled.
   const bool sampled = !ADJ && a.traces != nullptr;
   cluster_barrier();  // every level read, every mbarrier initialised
+  if (a.mute && rank == 0 && (need_dn || (tid >= svc && has_dn))) give_up();
 
   // The shot's source onto a vector of slab row r.
   auto add_source = [&](int r, int m, T (&o)[VZ]) {
@@ -669,7 +707,6 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
       asm volatile("" : "+r"(dpo), "+r"(dl), "+r"(first_cell));
       if (need_up) wait_halo(0, m);
       if (need_dn) wait_halo(1, m);
-      if (dead) cc[0][0] = T(NAN);
       const T* pc = buf + (m % NL) * BS + po0;
       const int level = (m + 1) % NL;
       T* pn = buf + level * BS + po0;
@@ -820,8 +857,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
         asm volatile("" : "+r"(dpo), "+r"(dl), "+r"(first_cell));
         if (need_up) wait_halo(0, m);
         if (need_dn) wait_halo(1, m);
-        if (dead) cc[0][0] = T(NAN);
-        const int level = (m + 1) % NL;
+          const int level = (m + 1) % NL;
         const T* pc = buf + (m % NL) * BS + po0;
         T* pn = buf + level * BS + po0;
         const int older = NL == 2 ? 0 : ((m + 2) % NL - level) * BS;
@@ -1048,7 +1084,8 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
     for (int m = 0; m < a.count; ++m) {
       const int n = ADJ ? a.n_first - m : a.n_first + m;
       const bool last = m + 1 == a.count, rec = phase == 0;
-      if (id == 0 && !last) {  // the next step's halos are expected
+      // the next step's halos are expected (after a wait that gave up, the phase before may not have completed)
+      if (id == 0 && !last && !*(volatile int*)&gave_up) {
         const unsigned tx = R * a.nv * 16, b = mbar_a + 8 * ((m + 1) & 1);
         if (has_up) mbar_expect(b, tx + (sampled ? 16 : 0));
         if (has_dn) mbar_expect(b + 16, tx);
@@ -1080,7 +1117,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
           if (has_dn && (n_edge > 0 || !last)) wait_halo(1, m);
           for (int e = id; e < n_edge; e += 32) sample(a.cap_list - 1 - e);
           __syncwarp();
-          if (id == 0 && has_dn && !last)
+          if (id == 0 && has_dn && !last && !dead)
             send_bytes(smem_addr(buf) + dn_off + a.nv * 16 + ((m + 1) % NL) * (unsigned)(BS * (int)sizeof(T)),
                        smem_addr(buf) - 16, 16, mbar_a + dn_off + 8 * ((m + 1) & 1));
         }
@@ -1101,6 +1138,11 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
   } else {
     steps(std::false_type{});
   }
+
+  if (*(volatile int*)&gave_up && tid < a.cluster)
+    asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(map_cta(smem_addr(&lost_sh), tid)), "r"(1) : "memory");
+  cluster_barrier();
+  const bool lost = *(volatile int*)&lost_sh != 0;
 
   // ---- the last two levels (and the gradient sums) back to memory
   if (work && (a.out_cur || ADJ)) {
@@ -1132,6 +1174,7 @@ __global__ void __launch_bounds__(resident_threads(PML), 1) resident2d(const __g
       if (X0 + rb == g.n0) store_row<T, VZ>(a.f_out[0] + so + cell0 + (long long)nr * ld, f_end, zc, g.n1);
     }
   }
+  if (lost) mark_lost<T, VZ, ADJ>(a, s, (long long)s * g.field + cell0, nr, dld, zc, g.n1);
   cluster_barrier();  // no CTA leaves while a neighbour may still address its shared memory
 }
 

@@ -51,6 +51,41 @@ std::atomic<unsigned long long> g_launches{0};
       return fail(NW_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e_)); \
   } while (0)
 
+// The words in which a kernel tells the host that a wait gave up, one per device, in pinned host memory so that the
+// host can look without synchronising (256 bytes, allocated at the first resident sweep and kept until the process
+// exits).
+constexpr int kReportDevices = 64;
+std::atomic<int*> g_reports{nullptr};
+int report_word(int** out) {
+  static std::mutex mu;
+  int dev = 0;
+  NW_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kReportDevices) return fail(NW_ERR_UNSUPPORTED, "device index above 63");
+  std::lock_guard<std::mutex> lock(mu);
+  int* words = g_reports.load();
+  if (!words) {  // in relaxed capture mode, so a first call inside a stream capture is safe too
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    NW_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaHostAlloc((void**)&words, kReportDevices * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+    NW_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    if (e != cudaSuccess) return fail(NW_ERR_CUDA, std::string("report words: ") + cudaGetErrorString(e));
+    std::fill(words, words + kReportDevices, 0);
+    g_reports.store(words);
+  }
+  *out = words + dev;
+  return NW_OK;
+}
+// What the current device has reported since last asked (no synchronisation).
+int take_report() {
+  int* words = g_reports.load();
+  if (!words) return NW_OK;
+  int dev = 0;
+  NW_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kReportDevices || !__atomic_load_n(words + dev, __ATOMIC_RELAXED)) return NW_OK;
+  if (!__atomic_exchange_n(words + dev, 0, __ATOMIC_RELAXED)) return NW_OK;
+  return fail(NW_ERR_TIMEOUT, "an earlier sweep on this device gave up waiting for a neighbouring CTA's rows; its results hold NaN");
+}
+
 int check_grid(const nw_grid* g) {
   if (!g) return fail(NW_ERR_ARG, "grid is NULL");
   if (g->ndim != 2 && g->ndim != 3) return fail(NW_ERR_UNSUPPORTED, "ndim must be 2 or 3");
@@ -283,6 +318,7 @@ struct TileCfg {  // one 2-D step kernel's tile: 8*rx rows by 32*vz columns, spc
 struct Tune {
   TileCfg fwd, adj;
   bool fwd_one = false, adj_one = false;  // one step per launch asked for (NW_TUNE_ONE_STEP_*)
+  bool mute = false;                      // NW_TUNE_MUTE
 };
 
 int check_tile(const nw_grid* g, const TileCfg& c, const char* which) {
@@ -311,7 +347,8 @@ int resolve_tune(const nw_grid* g, const nw_tuning* t, Tune* out) {
   // two forward steps per launch: 2-D grids without a PML (whose steps run a layer kernel beside the box)
   r.fwd.depth = (t && t->depth == 2 && g->ndim == 2 && g->absorbing != NW_ABS_PML) ? 2 : 1;
   if (t && (t->depth < 0 || t->depth > 2)) return fail(NW_ERR_ARG, "tuning.depth must be 0, 1 or 2");
-  if (t && (t->flags & ~(NW_TUNE_ONE_STEP_FORWARD | NW_TUNE_ONE_STEP_ADJOINT)) == 0) {
+  if (t && (t->flags & ~(NW_TUNE_ONE_STEP_FORWARD | NW_TUNE_ONE_STEP_ADJOINT | NW_TUNE_MUTE)) == 0) {
+    if (t->flags & NW_TUNE_MUTE) r.mute = true;
     r.fwd_one = (t->flags & NW_TUNE_ONE_STEP_FORWARD) != 0;
     r.adj_one = (t->flags & NW_TUNE_ONE_STEP_ADJOINT) != 0;
   }
@@ -520,6 +557,7 @@ struct ResidentPlan {
   bool pml = false;
   size_t smem = 0;
   double cost = 0.0;
+  bool mute = false;
 };
 
 template <typename T, int R, bool ADJ>
@@ -660,6 +698,7 @@ int resident_for(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
                           : resident_plan<T, 2, ADJ>(g, m, a->n_shots, n_imposed ? 0 : a->n_rec, a->n_cells, n_imposed, c, p);
   };
   int rc = plan(false);
+  p->mute = tu.mute;
   if (rc || !p->ok) return rc;
   // against one-step launches: cycles per step of the launch chain, or of the cells at the rate the tiled
   // kernels step them (16 shots of 552^2: 16.3 us forward, 18.1 us adjoint; with a PML 23.9 and 29.7 us)
@@ -670,7 +709,9 @@ int resident_for(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, 
     p->ok = false;
     return NW_OK;
   }
-  return crowded ? plan(true) : NW_OK;  // (the route is the one the problem takes alone)
+  if (crowded) rc = plan(true);  // (the route is the one the problem takes alone)
+  p->mute = tu.mute;
+  return rc;
 }
 
 template <typename T>
@@ -712,6 +753,7 @@ nw::Resident<T> resident_args(const nw_grid* g, const nw_medium* m, const nw_acq
   r.n_cells = a->n_cells;
   r.cap_list = p.cap_list;
   r.cap_ent = p.cap_ent;
+  r.mute = p.mute;
   return r;
 }
 
@@ -724,6 +766,8 @@ int resident_forward(const nw_grid* g, const nw::KGrid<T>& kg, const nw_medium* 
                      const nw_storage* snaps = nullptr, const int64_t* imposed = nullptr, int n_imposed = 0,
                      const T* imposed_tr = nullptr) {
   nw::Resident<T> r = resident_args<T>(g, m, a, t, p);
+  const int rc = report_word(&r.report);
+  if (rc) return rc;
   r.imposed = imposed;
   r.n_imposed = n_imposed;
   r.imposed_tr = imposed_tr;
@@ -762,6 +806,8 @@ int resident_adjoint(const nw_grid* g, const nw::KGrid<T>& kg, const nw_medium* 
                      const nw_time* t, const ResidentPlan& p, T* prev, T* cur, T* acc, int n, int n_last,
                      const T* gtr, const T* lap, int lap_n0, int lap_end, T* faces, cudaStream_t s) {
   nw::Resident<T> r = resident_args<T>(g, m, a, t, p);
+  const int rc = report_word(&r.report);
+  if (rc) return rc;
   if (p.pml)
     for (int ax = 0; ax < 2; ++ax) {  // step n reads parity n + 1 and writes parity n
       r.f_in[ax] = faces + (long long)(2 * ax + (n + 1) % 2) * r.level;
@@ -1598,6 +1644,7 @@ static bool misaligned16(const void* p) { return ((uintptr_t)p & 15u) != 0; }
 static int check_run(const nw_grid* g, const nw_medium* m, const nw_acquisition* a, const nw_time* t,
                      const nw_storage* st, const Tune& tu) {
   int rc = check_grid(g);
+  if (!rc) rc = take_report();
   if (rc) return rc;
   if (!m || !a || !t || !st) return fail(NW_ERR_ARG, "NULL descriptor");
   if (!m->c2dt2) return fail(NW_ERR_ARG, "medium.c2dt2 is NULL");
@@ -1824,16 +1871,19 @@ uint64_t nw_launch_count(void) { return g_launches.load(); }
 // Synchronises `stream`, returns and clears the sticky device status word (NW_OK if clean).
 int nw_status(void* stream) {
   NW_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  const int rc = take_report();
+  if (rc) return rc;
   int v = 0;
   NW_CUDA(cudaMemcpyFromSymbol(&v, nw::g_status, sizeof(int)));
   if (v) {
     const int zero = 0;
     NW_CUDA(cudaMemcpyToSymbol(nw::g_status, &zero, sizeof(int)));
-    return fail(v, v == NW_ERR_TIMEOUT ? "a wait for a neighbouring CTA's rows gave up"
-                                       : "a snapshot block held a non-finite value or scale");
+    return fail(v, "a snapshot block held a non-finite value or scale");
   }
   return NW_OK;
 }
+
+int nw_reported(void) { return take_report(); }
 
 }  // extern "C"
 

@@ -723,16 +723,23 @@ class GradientGraph:
         self._graph = graph
         torch.cuda.synchronize(self.device)
 
+    @_lib.on_device
     def replay(self) -> None:
         """Recompute ``loss`` and ``grad`` from the current ``c`` and ``observed`` (asynchronous; with
-        encoded snapshots, ``check()`` afterwards raises if a decode met a non-finite value)."""
+        encoded snapshots, ``check()`` afterwards raises if a decode met a non-finite value). Raises if an
+        earlier sweep on the device has reported that a wait inside it gave up."""
+        _lib.check(_lib.load().nw_reported())
         self._graph.replay()
 
+    @_lib.on_device
     def check(self) -> None:
-        """Synchronise and raise ``SolverError`` if a snapshot decode of the replays since the last
-        check met a non-finite value (no-op without encoded snapshots)."""
+        """With encoded snapshots, synchronise and raise ``SolverError`` if a snapshot decode of the replays
+        since the last check met a non-finite value. Raises, too, if a sweep has reported that a wait inside
+        it gave up (without encoded snapshots that is looked at without synchronising)."""
         if self.checks_status:
             _check_snapshot_status(_lib.stream_handle(self.device))
+        else:
+            _lib.check(_lib.load().nw_reported())
 
     def run(self, c: torch.Tensor, observed: torch.Tensor):
         """Check ``c`` like the operator does, copy both inputs in, replay and (with encoded snapshots)
