@@ -222,7 +222,9 @@ def autotune(ops: Sequence[WaveOperatorB200], *, steps: int = 120, device="cuda"
     each candidate's sweep on the device over a copy of the batch shortened in time: the longest
     problem to ``steps`` samples and every other one in proportion, so that the shortened batch runs
     the same mix of problems over its steps as the real one (the per-step cost of a problem does
-    not depend on the step count). Returns the 6-tuple tuning and the timings (seconds)."""
+    not depend on the step count). The shapes are those of the problems advanced together: where every
+    problem's sweeps take all their steps in one launch there is nothing to choose, and the first candidates
+    are returned. Returns the 6-tuple tuning and the timings (seconds)."""
     short = []
     n_t_max = max(op.n_t for op in ops)
     for op in ops:
@@ -259,6 +261,8 @@ def autotune(ops: Sequence[WaveOperatorB200], *, steps: int = 120, device="cuda"
         del bt
         return best
 
+    if all(any(op._plan(dev, dtype).sweep_route(op.n_sources, adj)[0] for adj in (False, True)) for op in short):
+        fwd_candidates, adj_candidates = fwd_candidates[:1], adj_candidates[:1]
     best_f = min(fwd_candidates, key=lambda t: results.setdefault(("fwd", t), sweep_time((*t, 0, 0, 0), "fwd")))
     best_a = min(adj_candidates,
                  key=lambda t: results.setdefault(("adj", t), sweep_time((*best_f, *t), "adj")))

@@ -501,8 +501,10 @@ class WaveOperatorB200(_LeapfrogB200):
         ``(vz, rx, shots_per_cta)`` with the forward chosen; depth 2 (two steps per launch) applies to
         2-D grids without a PML and falls back to one step elsewhere. Candidates the library refuses
         (a shape above the shared-memory limit, a float64 tile of four columns per thread) are
-        skipped. Sets ``self.tuning`` and returns it; ``self.autotune_results`` holds the microseconds
-        per step of each candidate. Traces are bitwise the same under every tuning; the gradient
+        skipped. A direction whose sweep takes all its steps in one launch (``DevicePlan.sweep_route``) has no
+        shape to choose: there only the first candidate of one step that the library
+        accepts and those of two are timed. Sets ``self.tuning`` and returns it; ``self.autotune_results`` holds the microseconds
+        per step of each candidate timed. Traces are bitwise the same under every tuning; the gradient
         regroups its float sums with the adjoint's shots per CTA."""
         self._validate(c)
         if len(self.domain.shape) != 2:
@@ -518,6 +520,8 @@ class WaveOperatorB200(_LeapfrogB200):
             # timed as graph replays, the way the gradient graphs and the batches run: eager sweeps
             # add the host's launch time per step, which differs between the layers (the PML's
             # side stream) and can rank the candidates differently
+            if tuning in results:
+                return results[tuning]
             short.tuning = tuning
             short._plans.clear()
             fwd = adj = math.inf
@@ -541,8 +545,16 @@ class WaveOperatorB200(_LeapfrogB200):
 
         fwd_c = fwd_candidates or self.FWD_CANDIDATES
         adj_c = adj_candidates or self.ADJ_CANDIDATES
+        plan = short._plan(c.device, c.dtype)
+        S = min(short.n_sources, short.source_batch or short.n_sources)
+        if plan.sweep_route(S)[0]:  # every shape of one step per launch would run the same kernel
+            one = next((f for f in fwd_c if f[3] != 2 and per_step((*f[:3], 0, 0, 0, f[3]))[0] < math.inf), None)
+            fwd_c = [f for f in fwd_c if f[3] == 2 or f == one] or fwd_c
         best_f = min(fwd_c, key=lambda f: per_step((*f[:3], 0, 0, 0, f[3]))[0])
-        best_a = min(adj_c, key=lambda a: per_step((*best_f[:3], *a, best_f[3]))[1])
+        adj_key = lambda a: per_step((*best_f[:3], *a, best_f[3]))[1]  # noqa: E731
+        if plan.sweep_route(S, adjoint=True)[0]:
+            adj_c = [next((a for a in adj_c if adj_key(a) < math.inf), adj_c[0])]
+        best_a = min(adj_c, key=adj_key)
         if math.isinf(results.get((*best_f[:3], *best_a, best_f[3]), (math.inf, math.inf))[1]):
             raise ConfigError("autotune: the library refused every candidate launch shape")
         self.tuning = (*best_f[:3], *best_a, best_f[3])

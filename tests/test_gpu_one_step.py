@@ -6,16 +6,13 @@ step per launch (``nw_tuning.flags``), and the two ways are compared with each o
 
 from __future__ import annotations
 
-import ctypes as C
-
-import numpy as np
 import pytest
 import torch
 
 from conftest import cotangent, load_golden, rel_l2
 from nefi_b200 import WaveOperatorB200, _lib
 from nefi_b200._compat import Domain
-from nefi_b200.batched import BatchedFWI
+from nefi_b200.batched import BatchedFWI, autotune
 from nefi_b200.plan import DevicePlan
 from test_gpu_batched import (  # noqa: F401  (collected here, under the fixture below)
     _problem,
@@ -142,3 +139,24 @@ def test_a_flag_that_is_none_counts_as_no_flag(cuda_device):
         assert (plan.sweep_route(2), plan.sweep_route(2, adjoint=True)) == want
     plan.set_tuning(flags=_lib.ONE_STEP_ADJOINT)
     assert plan.sweep_route(2) == want[0] and plan.sweep_route(2, adjoint=True) == (0, 0)
+
+
+def test_the_autotuners_time_only_what_can_be_chosen(cuda_device):
+    """A direction whose sweep takes all its steps in one launch runs the same kernel under every shape."""
+    op = _layered_op(shots=4, n_t=21)
+    c = torch.full(op.domain.shape, 2400.0, device=cuda_device)
+    plan = op._plan(cuda_device, torch.float32)
+    assert plan.sweep_route(4)[0] and plan.sweep_route(4, adjoint=True)[0]
+    tu = op.autotune(c, steps=20, repeats=1)
+    assert {k[:3] for k in op.autotune_results if k[6] == 1} == {op.FWD_CANDIDATES[0][:3]}
+    assert {k[3:6] for k in op.autotune_results} == {(0, 0, 0), op.ADJ_CANDIDATES[0]} and len(tu) == 7
+    op64 = _layered_op(shots=4, n_t=21)  # (float64 takes no tile of four columns a thread)
+    assert op64.autotune(c.double(), steps=20, repeats=1)[0] == 2
+    large = _layered_op(n=600, shots=9, n_t=11)
+    large.autotune(torch.full(large.domain.shape, 2400.0, device=cuda_device), steps=10, repeats=1)
+    assert len(large.autotune_results) >= len(op.FWD_CANDIDATES) + len(op.ADJ_CANDIDATES)
+    small = [_problem(n, 2, 31, n)[0] for n in (40, 56)]
+    tuning, times = autotune(small, steps=20, device=cuda_device, repeats=1)
+    assert len(times) == 2 and all(v > 0 for v in tuning)
+    mixed = small + [_problem(632, 9, 24, 1)[0]]
+    assert len(autotune(mixed, steps=20, device=cuda_device, repeats=1)[1]) == 10
