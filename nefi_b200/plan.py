@@ -500,15 +500,17 @@ def binomial_steps(n_steps: int, k: int, n_slots: int) -> int:
 
 def plan_storage(plan: DevicePlan, n_shots: int, n_steps: int, grad_mode: str,
                  checkpoint_every: int | None, snapshot: str, budget: int | None,
-                 checkpoint_slots: int | None = None):
+                 checkpoint_slots: int | None = None, held: int = 0):
     """Choose the wavefield storage of a gradient run: ``("history",)``, ``("checkpoint", K)``
     (segments of ``K`` steps, a snapshot per segment start) or ``("checkpoint", K, slots)`` (binomial
     checkpointing of the segments over ``slots`` snapshot slots, fewer than the segments).
 
     ``grad_mode="autograd"`` keeps every level when it fits ``budget`` bytes and otherwise
     checkpoints; ``"checkpoint"`` with exact snapshots and no segment length or slot count asked for keeps
-    every level, too, when that takes no more than an eighth of the budget (the gradient is bitwise the
-    same and a third of its steps, the recomputation, falls away), and otherwise uses segments of ``checkpoint_every`` steps (default
+    every level, too, while such histories, the ``held`` bytes of those already alive included, take no more
+    than an eighth of the budget (the gradient is bitwise the same and a third of its steps, the recomputation,
+    falls away; the eighth is what the default mode may take of a program's memory beyond its
+    ``O(sqrt(n_steps))`` levels, a choice and not a measured optimum), and otherwise uses segments of ``checkpoint_every`` steps (default
     ``ceil(sqrt(n_steps))``, the reference's choice) or the shortest segment whose storage fits the
     budget. When no segment length lets a snapshot per segment fit, the segment length and slot count
     that fit and need the fewest forward steps are chosen (binomial checkpointing, whose extra forward
@@ -518,7 +520,7 @@ def plan_storage(plan: DevicePlan, n_shots: int, n_steps: int, grad_mode: str,
     hist = (n_steps + 3) * lvl  # n_steps Lap p levels and the pressure ring
     if grad_mode == "autograd" and (budget is None or hist <= budget) and not checkpoint_slots:
         return ("history", None)
-    if snapshot == "exact" and budget is not None and 8 * hist <= budget and not (checkpoint_every or checkpoint_slots):
+    if snapshot == "exact" and budget is not None and 8 * (hist + held) <= budget and not (checkpoint_every or checkpoint_slots):
         return ("history", None)
     kind = _lib.SNAP_KINDS[snapshot]
     extra = 4 * lvl if plan.pml is not None else 0  # the PML's face fields
