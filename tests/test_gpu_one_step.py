@@ -78,31 +78,58 @@ def _gradient(op, c, g, flags):
     return tr.detach(), gc, int(_lib.load().nw_launch_count() - n0)
 
 
+def _both_ways(shape, shots, absorbing, order, dtype, dev, width=8):
+    """A resident gradient against that of one-step launches: traces bitwise, the gradient up to the order of its sums
+    (the tolerances of the launch-shape test). Returns the rows a thread steps, forward and adjoint."""
+    h = 10.0
+    n0, n1 = shape
+    src = [[(k + 0.4) * n0 * h / shots, (0.2 + 0.6 * k / shots) * n1 * h] for k in range(shots)]
+    rec = [[(i + 0.5) * h, (0.2 + 0.6 * (i * shots // n0) / shots) * n1 * h + (-1) ** i * 1.3 * h] for i in range(n0)]
+    op = WaveOperatorB200(Domain(shape, ((0.0, n0 * h), (0.0, n1 * h))), src, rec, n_t=24, dt_obs=2.2e-3, f0=60.0,
+                          c_max=2600.0, order=order, absorbing=absorbing, absorb_width=width * h, grad_mode="autograd")
+    x = torch.linspace(0, 1, n0, dtype=torch.float64)[:, None]
+    z = torch.linspace(0, 1, n1, dtype=torch.float64)[None, :]
+    c = (2000.0 + 400.0 * z + 120.0 * torch.sin(9 * x + 4 * z)).to(dtype).to(dev)
+    g = torch.tensor(cotangent((shots, len(rec), 24), 3), dtype=dtype, device=dev)
+    tr0, g0, n_one = _gradient(op, c, g, ONE_STEP)
+    assert n_one >= 2 * op.n_steps
+    tr1, g1, n_many = _gradient(op, c, g, 0)
+    plan = op._plan(dev, dtype)
+    fwd, adj = plan.sweep_route(shots), plan.sweep_route(shots, adjoint=True)
+    assert fwd[0] > 0 or adj[0] > 0
+    assert n_many < 20 + op.n_steps * ((fwd[0] == 0) + (adj[0] == 0)) * (2 if absorbing == "pml" else 1)
+    loud = float(tr0.abs().max())
+    same = torch.equal(tr0, tr1)
+    assert same and loud > 0
+    assert rel_l2(g1.cpu().numpy(), g0.cpu().numpy()) < (1e-12 if dtype == torch.float64 else 1e-5)
+    return fwd[1], adj[1]
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 @pytest.mark.parametrize("order", [2, 4])
 @pytest.mark.parametrize("absorbing", ["none", "sponge", "cerjan", "pml"])
 @pytest.mark.parametrize("shape,shots", [((50, 47), 3), ((130, 61), 5), ((203, 200), 6)])
 def test_resident_gradient_is_that_of_one_step_launches(shape, shots, absorbing, order, dtype, cuda_device):
-    """Traces bitwise; the gradient up to the order of its sums (the tolerances of the launch-shape test)."""
-    h = 10.0
-    n0, n1 = shape
-    src = [[(k + 0.4) * n0 * h / shots, (0.2 + 0.1 * k) * n1 * h] for k in range(shots)]
-    rec = [[(i + 0.5) * h, (0.2 + 0.1 * (i * shots // n0)) * n1 * h + (-1) ** i * 1.3 * h] for i in range(n0)]
-    op = WaveOperatorB200(Domain(shape, ((0.0, n0 * h), (0.0, n1 * h))), src, rec, n_t=24, dt_obs=2.2e-3, f0=60.0,
-                          c_max=2600.0, order=order, absorbing=absorbing, absorb_width=8 * h, grad_mode="autograd")
-    x = torch.linspace(0, 1, n0, dtype=torch.float64)[:, None]
-    z = torch.linspace(0, 1, n1, dtype=torch.float64)[None, :]
-    c = (2000.0 + 400.0 * z + 120.0 * torch.sin(9 * x + 4 * z)).to(dtype).to(cuda_device)
-    g = torch.tensor(cotangent((shots, len(rec), 24), 3), dtype=dtype, device=cuda_device)
-    tr0, g0, n_one = _gradient(op, c, g, ONE_STEP)
-    assert n_one >= 2 * op.n_steps
-    tr1, g1, n_many = _gradient(op, c, g, 0)
-    plan = op._plan(cuda_device, dtype)
-    assert plan.sweep_route(shots)[0] > 0 and plan.sweep_route(shots, adjoint=True)[0] > 0 and n_many < 20
-    loud = float(tr0.abs().max())
-    same = torch.equal(tr0, tr1)
-    assert same and loud > 0
-    assert rel_l2(g1.cpu().numpy(), g0.cpu().numpy()) < (1e-12 if dtype == torch.float64 else 1e-5)
+    rows = _both_ways(shape, shots, absorbing, order, dtype, cuda_device)
+    assert all(rows) or shape[0] > 200
+
+
+# (layer, cells a side, shots, dtype, rows a thread steps forward and adjoint at order 4; 0: not looked at here)
+TALL = [("none", 200, 16, torch.float32, 6, 6), ("none", 256, 16, torch.float32, 8, 8),
+        ("sponge", 256, 16, torch.float32, 12, 12), ("sponge", 400, 16, torch.float32, 12, 0),
+        ("sponge", 200, 1, torch.float64, 6, 0), ("sponge", 168, 1, torch.float64, 0, 6),
+        ("sponge", 128, 16, torch.float64, 8, 8), ("sponge", 168, 16, torch.float64, 12, 12),
+        ("pml", 168, 16, torch.float32, 6, 0), ("pml", 256, 1, torch.float32, 6, 6),
+        ("pml", 100, 16, torch.float64, 6, 0), ("pml", 168, 1, torch.float64, 0, 6)]
+
+
+@pytest.mark.parametrize("order", [2, 4])
+@pytest.mark.parametrize("absorbing,n,shots,dtype,fwd,adj", TALL)
+def test_tall_strips(absorbing, n, shots, dtype, fwd, adj, order, cuda_device):
+    """Strips of six rows a thread and more (twelve: the adjoint streams c^2 dt^2), as grids of 300^2 and up take."""
+    rows = _both_ways((n, n), shots, absorbing, order, dtype, cuda_device, width=20)
+    if order == 4:
+        assert all(w in (0, r) for w, r in zip((fwd, adj), rows)), rows
 
 
 @pytest.mark.parametrize("absorbing", ["sponge", "pml"])
