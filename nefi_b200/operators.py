@@ -687,7 +687,7 @@ class _PATFunction(torch.autograd.Function):
         _forward_sweep(plan, medium, acq, run, 0, op.n_steps, traces, stream)
         if needs_grad:
             ctx.op, ctx.plan, ctx.S, ctx.batch, ctx.c2dt2, ctx.p0_level = op, plan, S, batch, c2dt2, p0_level
-            ctx.run = run if keep else None
+            ctx.run, ctx.keep = run if keep else None, keep
             ctx.save_for_backward(c)
         if not keep:
             run.release()
@@ -699,6 +699,8 @@ class _PATFunction(torch.autograd.Function):
     def backward(ctx, grad_traces: torch.Tensor):
         (c,) = ctx.saved_tensors
         op, run, S, plan = ctx.op, ctx.run, ctx.S, ctx.plan
+        if ctx.keep and run is None:
+            raise OperatorError("a second backward through this call: the first released its stored wavefield")
         dev = grad_traces.device
         stream = _lib.stream_handle(dev)
         lib = _lib.load()
