@@ -2141,6 +2141,14 @@ int batch_solos(const nw_batch_problem* P, const std::vector<char>& solo, cudaSt
     return rest();
   });
 }
+// The storage of a problem that runs apart, without what the batched calls ignore: a schedule and a fourth ring level.
+nw_storage batch_storage(const nw_batch_problem& q) {
+  nw_storage st = q.storage;
+  st.snap_slot = st.schedule = nullptr;
+  st.n_schedule = 0;
+  st.ring_levels = 3;
+  return st;
+}
 template <typename T>
 int batch_solo_flags(const nw_batch_problem* P, int n, const Tune& tu, std::vector<char>* solo) {
   solo->assign(n, 0);
@@ -2366,7 +2374,8 @@ int batch_forward_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
   };
   return batch_solos(P, solo, s,
                      [&](const nw_batch_problem& q, cudaStream_t lane) {
-                       return forward_impl<T>(&q.grid, &q.medium, &q.acq, &q.time, &q.storage, tu, 0, q.time.n_steps,
+                       const nw_storage st = batch_storage(q);
+                       return forward_impl<T>(&q.grid, &q.medium, &q.acq, &q.time, &st, tu, 0, q.time.n_steps,
                                               (T*)q.traces, lane, true);
                      },
                      rest);
@@ -2447,7 +2456,8 @@ int batch_adjoint_impl(const nw_batch_problem* P, int n, const Tune& tu, const v
   };
   return batch_solos(P, solo, s,
                      [&](const nw_batch_problem& q, cudaStream_t lane) {
-                       return adjoint_impl<T>(&q.grid, &q.medium, &q.acq, &q.time, &q.storage, tu, (const T*)q.grad_traces,
+                       const nw_storage st = batch_storage(q);
+                       return adjoint_impl<T>(&q.grid, &q.medium, &q.acq, &q.time, &st, tu, (const T*)q.grad_traces,
                                               (T*)q.work, (T*)q.grad_acc, (T*)nullptr, (T*)nullptr, lane, true);
                      },
                      rest);
