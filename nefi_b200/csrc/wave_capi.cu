@@ -568,9 +568,14 @@ int resident_plan(const nw_grid* g, const nw_medium* m, int n_shots, int n_rec, 
   const bool pml = g->absorbing == NW_ABS_PML;
   const int levels = pml && ADJ ? 3 : 2;
   const int n0 = g->n[0], nv = (g->n[1] + L::VZ - 1) / L::VZ;
-  const int x0 = pml ? m->pml_core[0] : g->core_lo[0], x1 = pml ? m->pml_core[1] : g->core_hi[0];
-  const int z0 = pml ? m->pml_core[2] : g->core_lo[1], z1 = pml ? m->pml_core[3] : g->core_hi[1];
-  if (x0 < 0 || z0 < 0 || x1 < x0 || z1 < z0 || x1 > n0 || z1 > g->n[1]) return fail(NW_ERR_ARG, "medium.pml_core lies outside the grid");
+  int x0 = 0, x1 = n0, z0 = 0, z1 = g->n[1];
+  if (pml) {
+    x0 = m->pml_core[0]; x1 = m->pml_core[1]; z0 = m->pml_core[2]; z1 = m->pml_core[3];
+    if (x0 < 0 || z0 < 0 || x1 < x0 || z1 < z0 || x1 > n0 || z1 > g->n[1]) return fail(NW_ERR_ARG, "medium.pml_core lies outside the grid");
+  } else if (g->absorbing != NW_ABS_NONE) {  // (a core beyond the grid, or none, is no error)
+    x0 = std::min(std::max((int)g->core_lo[0], 0), n0); x1 = std::min(std::max((int)g->core_hi[0], x0), n0);
+    z0 = std::min(std::max((int)g->core_lo[1], 0), z1); z1 = std::min(std::max((int)g->core_hi[1], z0), z1);
+  }
   int edge_lo = (z0 + L::VZ - 1) / L::VZ, edge_hi = z1 / L::VZ;
   if (edge_lo >= edge_hi || g->absorbing == NW_ABS_NONE) edge_lo = 0, edge_hi = g->absorbing == NW_ABS_NONE ? nv : 0;
   const int ne = edge_lo + nv - edge_hi;
