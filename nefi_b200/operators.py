@@ -183,18 +183,21 @@ _histories_lock = threading.Lock()
 _history_key = itertools.count()
 
 
-def _hold_history(owner, device: torch.device, nbytes: int) -> None:
+def _hold_history(owner, plan: DevicePlan, device: torch.device, nbytes: int) -> None:
     """Count ``nbytes`` of wavefield history on ``device`` for as long as ``owner`` lives or until it sets
     ``history_bytes`` to 0."""
-    owner.history_bytes, owner.history_device = nbytes, torch.device(device)
+    owner.history_bytes, owner.history_device, owner.history_plan = nbytes, torch.device(device), plan
     with _histories_lock:
         _histories[next(_history_key)] = owner
 
 
-def _held_history(device: torch.device) -> int:
+def _held_history(op: "_LeapfrogB200", plan: DevicePlan, device: torch.device) -> int:
+    """Bytes of the histories alive that share the budget of ``op``: all on the device, of this operator's plan
+    alone if it has a ``memory_budget`` of its own."""
     with _histories_lock:
         owners = list(_histories.values())
-    return sum(o.history_bytes for o in owners if o.history_device == device)
+    return sum(o.history_bytes for o in owners
+               if o.history_device == device and (op.memory_budget is None or o.history_plan is plan))
 
 
 class _Run:
@@ -220,7 +223,7 @@ class _Run:
             # (the adjoint multiplies them only into sums of cells outside the grid, never stored)
             self.history = plan.empty_levels(n_steps, n_shots, zero=False)
             self.storage.history = self.history.data_ptr()
-            _hold_history(self, self.history.device, self.history.numel() * self.history.element_size())
+            _hold_history(self, plan, self.history.device, self.history.numel() * self.history.element_size())
         elif self.kind == "checkpoint":
             k = int(mode[1])
             kind = _lib.SNAP_KINDS[snapshot]
@@ -316,7 +319,7 @@ class _FWIFunction(torch.autograd.Function):
         needs_grad = ctx.needs_input_grad[0]
         mode = (plan_storage(plan, n_shots, op.n_steps, op.grad_mode, op.checkpoint_every,
                              op.snapshot, op._budget(c.device), op.checkpoint_slots,
-                             _held_history(c.device)) if needs_grad else ("ring", None))
+                             _held_history(op, plan, c.device)) if needs_grad else ("ring", None))
         op.last_storage = tuple(mode)
         run = _Run(plan, n_shots, op.n_steps, mode, op.snapshot)
         traces = torch.empty(n_shots, plan.n_rec, op.n_t, device=c.device, dtype=c.dtype)
@@ -361,7 +364,8 @@ class WaveOperatorB200(_LeapfrogB200):
     1.8e-4, 2.0e-3 and 1.7e-2 on a 128^2, 1000-step case) and ``memory_budget`` (bytes available for
     wavefield storage; default 85 % of the device memory that is free or held unused by PyTorch's
     allocator). The default ``grad_mode="checkpoint"`` stores all levels from forward to backward while such
-    histories, those of other live graphs on the device included, take no more than an eighth of that budget:
+    histories, those of other live graphs on the device included (of this operator's, given a ``memory_budget``),
+    take no more than an eighth of that budget:
     the same gradient without the recomputation; give ``checkpoint_every`` (the reference's default is
     ``ceil(sqrt(n_steps))``) for checkpoints in any case. ``last_storage`` tells which it was.
     Output ``(n_sources, n_receivers, n_t)`` at ``t_j = j dt_obs``; the gradient w.r.t. ``c`` is
@@ -457,7 +461,7 @@ class WaveOperatorB200(_LeapfrogB200):
         plan = self._plan(c.device, c.dtype)
         n = self.n_sources
         chunk = self.source_batch or n
-        budget, held = self._budget(c.device), _held_history(c.device)
+        budget, held = self._budget(c.device), _held_history(self, plan, c.device)
         return [plan_storage(plan, min(n, s0 + chunk) - s0, self.n_steps, self.grad_mode, self.checkpoint_every,
                              self.snapshot, budget, self.checkpoint_slots, held) for s0 in range(0, n, chunk)]
 
@@ -678,7 +682,7 @@ class _PATFunction(torch.autograd.Function):
         keep = need_c or (needs_grad and bool(op.checkpoint_every or op.checkpoint_slots))
         mode = (plan_storage(plan, S, op.n_steps, op.grad_mode, op.checkpoint_every, op.snapshot,
                              op._budget(p0.device), op.checkpoint_slots,
-                             _held_history(p0.device)) if keep else ("ring", None))
+                             _held_history(op, plan, p0.device)) if keep else ("ring", None))
         run = _Run(plan, S, op.n_steps, mode, op.snapshot)
         _lib.check(lib.nw_initial_state(C.byref(plan.g), plan.n_abs, C.byref(medium), S, p0f.data_ptr(),
                                         run.level(-1).data_ptr(), run.level(0).data_ptr(), stream))
@@ -765,8 +769,9 @@ class GradientGraph:
         self._graph = graph
         plan, n, chunk = op._plan(self.device, self.c.dtype), op.n_sources, op.source_batch or op.n_sources
         # the chunks run one after the other in the graph's own memory
-        _hold_history(self, self.device, max(op.n_steps * plan.level_bytes(min(n - s0, chunk)) if mode[0] == "history" else 0
-                                             for s0, mode in zip(range(0, n, chunk), self._modes)))
+        _hold_history(self, plan, self.device,
+                      max(op.n_steps * plan.level_bytes(min(n - s0, chunk)) if mode[0] == "history" else 0
+                          for s0, mode in zip(range(0, n, chunk), self._modes)))
         torch.cuda.synchronize(self.device)
 
     @_lib.on_device

@@ -96,3 +96,17 @@ def test_histories_alive_count_against_the_eighth(cuda_device):
     del first
     op.gradient_graph(c.detach(), obs)
     assert op.last_storage == ("history", None)
+
+
+@pytest.mark.gpu
+def test_an_operators_own_budget_counts_its_own_histories(cuda_device):
+    case = load_golden("fwi_o4_sponge")
+    c = torch.tensor(case["c"], dtype=torch.float32, device=cuda_device, requires_grad=True)
+    other = make_op(case)({"c": c})  # a history alive on the device
+    op = make_op(case, grad_mode="checkpoint")
+    op.memory_budget = 8 * _hist(op, cuda_device, torch.float32, op.n_sources)
+    tr = op({"c": c})
+    assert op.last_storage == ("history", None)
+    op({"c": c})
+    assert op.last_storage[0] == "checkpoint"
+    del other, tr
